@@ -453,7 +453,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
       }
     std::vector<double> values;
     std::vector<C64> vectors;
-    device_hermitian_eigen(size, P, values, vectors, c.ops.stream());
+    device_hermitian_eigen(size, P, values, vectors, c.ops);
     const int active = k - l;
     const int keep = keep_for(active);
     const std::vector<size_t> indices = select_indices(values, o.target, std::min(keep, size));
@@ -544,7 +544,7 @@ EigshResult dense_eigsh(Ctx& c, const EigshOptions& o) {
       if (std::abs(dense[r * n + col] - std::conj(dense[col * n + r])) > 1.0e-12) raise(QMBED_NON_HERMITIAN, "");
   std::vector<double> values;
   std::vector<C64> vectors;
-  device_hermitian_eigen(static_cast<int>(n), dense, values, vectors, c.ops.stream());
+  device_hermitian_eigen(static_cast<int>(n), dense, values, vectors, c.ops);
   std::vector<size_t> order(n);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return values[a] < values[b]; });

@@ -375,7 +375,7 @@ class BlockSolver {
   void orthonormalize(int prec, void*& A, void*& B, int passes) {
     for (int pass = 0; pass < passes; ++pass) {
       std::vector<double> G = gram(prec, A, A), mu, V;
-      device_symmetric_eigen(nb_, G, mu, V, ops_.stream());
+      device_symmetric_eigen(nb_, G, mu, V, ops_);
       const double top = std::max(mu.back(), std::numeric_limits<double>::min());
       const double floor = top * (prec == 64 ? 1.0e-28 : 1.0e-14);
       std::vector<double> C(static_cast<size_t>(nb_) * nb_);
@@ -391,7 +391,7 @@ class BlockSolver {
   void rayleigh_ritz(int prec, void*& A, void*& B, void* W, std::vector<double>& theta, std::vector<double>& res) {
     act(prec, A, nullptr, W, 1.0, 0.0, 0.0);
     std::vector<double> Tm = gram(prec, A, W), Y;
-    device_symmetric_eigen(nb_, Tm, theta, Y, ops_.stream());
+    device_symmetric_eigen(nb_, Tm, theta, Y, ops_);
     std::vector<double> r2 = rotate(prec, A, B, W, Y, theta, true);
     std::swap(A, B);
     res.assign(nb_, 0.0);

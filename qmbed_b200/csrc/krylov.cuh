@@ -102,16 +102,17 @@ class BlockOps {
 void tridiagonal_eigen(std::vector<double> diag, std::vector<double> off, bool first_row, std::vector<double>& values,
                        std::vector<double>& V);
 
-// Eigen-decomposition of a small dense Hermitian matrix (row-major, n <= 2048)
-// by parallel cyclic Jacobi in one CTA. Values are returned unsorted with
-// column-major eigenvectors.
+// Eigen-decomposition of a small dense Hermitian matrix (row-major, n <= 1024)
+// by parallel cyclic Jacobi in one CTA, in shared memory while it fits. Values
+// are returned unsorted with column-major eigenvectors. Work buffer: a
+// workspace slot of `ops`.
 void device_hermitian_eigen(int n, const std::vector<C64>& a, std::vector<double>& values, std::vector<C64>& vectors,
-                            cudaStream_t stream);
+                            BlockOps& ops);
 
 // Ascending eigenpairs of a real symmetric m x m matrix (row-major; the
 // symmetric part is used) by the same device Jacobi, with real eigenvectors
 // as the columns of V (row-major V[i * m + j]).
 void device_symmetric_eigen(int m, const std::vector<double>& a, std::vector<double>& values, std::vector<double>& V,
-                            cudaStream_t stream);
+                            BlockOps& ops);
 
 }  // namespace qmbed

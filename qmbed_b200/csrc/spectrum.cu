@@ -48,7 +48,7 @@ std::vector<double> spectral_function(const LinearOperatorView& view, const doub
       for (uint64_t c = 0; c < n; ++c)
         if (std::abs(dense[r * n + c] - std::conj(dense[c * n + r])) > 1.0e-12) raise(QMBED_NON_HERMITIAN, "");
     std::vector<C64> vectors;
-    device_hermitian_eigen(static_cast<int>(n), dense, energies, vectors, ops.stream());
+    device_hermitian_eigen(static_cast<int>(n), dense, energies, vectors, ops);
     std::vector<C64> v(static_cast<size_t>(n));
     QMBED_CUDA(cudaMemcpyAsync(v.data(), created, n * 16, cudaMemcpyDeviceToHost, ops.stream()));
     ops.sync();
