@@ -111,6 +111,118 @@ struct ChainBuilder {
 
 }  // namespace
 
+// One product in flip form; false when it repeats a site or holds a factor
+// without one (the digit then changes between factors).
+static bool flip_form(const Instance& a, const LocalFactors& f, uint64_t* flip, TermKey* key, C64* k) {
+  uint64_t seen = 0, flips = 0, req_mask = 0, req_val = 0, sign_mask = 0;
+  C64 c(a.cr, a.ci);
+  for (int q = 0; q < a.n; ++q) {
+    const char sym = a.sym[q];
+    if (sym == 'I') continue;
+    const uint64_t bit = 1ull << a.site[q];
+    if (seen & bit) return false;
+    seen |= bit;
+    switch (sym) {
+      case 'z':
+        sign_mask |= bit;
+        c *= f.z[1];
+        break;
+      case '+':
+        flips |= bit;
+        req_mask |= bit;
+        c *= f.raise;
+        break;
+      case '-':
+        flips |= bit;
+        req_mask |= bit;
+        req_val |= bit;
+        c *= f.lower;
+        break;
+      case 'x':
+        flips |= bit;
+        c *= f.xy_scale * f.raise;
+        break;
+      case 'y':
+        // (d ? +i : -i) * g: i g times the sign of the digit
+        flips |= bit;
+        sign_mask |= bit;
+        c *= C64(0.0, f.xy_scale * f.raise);
+        break;
+      default:
+        return false;
+    }
+  }
+  *flip = flips;
+  *key = {req_mask, req_val, sign_mask};
+  // the row entry is conj(coefficient * amplitude)
+  *k = std::conj(c);
+  return true;
+}
+
+bool hermitian_by_terms(const std::vector<Instance>& adjoint, const std::vector<Instance>& forward,
+                        const LocalFactors& f, int sites) {
+  if (sites > 64 || f.z[0] != -f.z[1] || f.raise != f.lower) return false;
+  struct Sum {
+    C64 k;
+    double abs = 0.0;
+    int count = 0;
+  };
+  std::map<uint64_t, std::map<TermKey, Sum>> sides[2];
+  for (int side = 0; side < 2; ++side)
+    for (const Instance& a : side == 0 ? adjoint : forward) {
+      uint64_t flip;
+      TermKey key;
+      C64 k;
+      if (!flip_form(a, f, &flip, &key, &k)) return false;
+      Sum& s = sides[side][flip][key];
+      s.k += k;
+      s.abs += std::abs(k);
+      ++s.count;
+    }
+  // the same coefficients on both sides
+  for (int side = 0; side < 2; ++side)
+    for (const auto& [flip, terms] : sides[side]) {
+      const auto other = sides[1 - side].find(flip);
+      for (const auto& [key, s] : terms) {
+        C64 k(0.0, 0.0);
+        if (other != sides[1 - side].end()) {
+          const auto it = other->second.find(key);
+          if (it != other->second.end()) k = it->second.k;
+        }
+        if (s.k != k) return false;
+      }
+    }
+  // Largest sum one row can hold: products that ask for different digits of
+  // the same sites exclude one another.
+  double row_abs = 0.0, row_terms = 0.0;
+  size_t targets = 0;
+  for (const auto& [flip, terms] : sides[0]) {
+    std::map<uint64_t, std::map<uint64_t, std::pair<double, int>>> by_digits;
+    for (const auto& [key, s] : terms) {
+      auto& d = by_digits[std::get<0>(key)][std::get<1>(key)];
+      d.first += s.abs;
+      d.second += s.count;
+    }
+    for (const auto& [mask, values] : by_digits) {
+      double abs = 0.0;
+      int count = 0;
+      for (const auto& [value, d] : values) {
+        abs = std::max(abs, d.first);
+        count = std::max(count, d.second);
+      }
+      row_abs += abs;
+      row_terms += count;
+    }
+    targets += flip != 0 ? 1 : 0;
+  }
+  // A row's sum of m terms of total size S is off by at most (m - 1) u S in
+  // either order; a target on the row's own representative joins the
+  // diagonal, so both kinds count together.
+  constexpr double kUnit = 1.1102230246251565e-16;
+  if (!(2.0 * (row_terms + 4.0) * kUnit * row_abs < 0.5e-12)) return false;
+  return targets <= 128;  // more distinct transitions than this are refused by the row expansion
+}
+
 FlipProgram compile_flip_program(const std::vector<Instance>& adjoint, const LocalFactors& f, int sites,
                                  bool fixed_weight) {
   FlipProgram prog;
@@ -119,47 +231,12 @@ FlipProgram compile_flip_program(const std::vector<Instance>& adjoint, const Loc
   if (f.z[0] != -f.z[1] || f.raise != f.lower) return prog;
   std::map<uint64_t, std::map<TermKey, C64>> by_flip;
   for (const Instance& a : adjoint) {
-    uint64_t seen = 0, flip = 0, req_mask = 0, req_val = 0, sign_mask = 0;
-    C64 k(a.cr, a.ci);
-    for (int q = 0; q < a.n; ++q) {
-      const char sym = a.sym[q];
-      if (sym == 'I') continue;
-      const uint64_t bit = 1ull << a.site[q];
-      if (seen & bit) return FlipProgram{};  // a repeated site: the digit changes between factors
-      seen |= bit;
-      switch (sym) {
-        case 'z':
-          sign_mask |= bit;
-          k *= f.z[1];
-          break;
-        case '+':
-          flip |= bit;
-          req_mask |= bit;
-          k *= f.raise;
-          break;
-        case '-':
-          flip |= bit;
-          req_mask |= bit;
-          req_val |= bit;
-          k *= f.lower;
-          break;
-        case 'x':
-          flip |= bit;
-          k *= f.xy_scale * f.raise;
-          break;
-        case 'y':
-          // (d ? +i : -i) * g: i g times the sign of the digit
-          flip |= bit;
-          sign_mask |= bit;
-          k *= C64(0.0, f.xy_scale * f.raise);
-          break;
-        default:
-          return FlipProgram{};
-      }
-    }
+    uint64_t flip;
+    TermKey key;
+    C64 k;
+    if (!flip_form(a, f, &flip, &key, &k)) return FlipProgram{};
     if (k == C64(0.0, 0.0)) continue;
-    // the row entry is conj(coefficient * amplitude)
-    by_flip[flip][{req_mask, req_val, sign_mask}] += std::conj(k);
+    by_flip[flip][key] += k;
   }
   // Products whose amplitude depends on at most two sites (those they flip
   // included) become 4-entry amplitude tables indexed by the two digits.

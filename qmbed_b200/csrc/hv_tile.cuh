@@ -99,6 +99,14 @@ struct FlipProgram {
 FlipProgram compile_flip_program(const std::vector<Instance>& adjoint, const LocalFactors& f, int sites,
                                  bool fixed_weight);
 
+// True when the adjoint and the forward products have the same flip form,
+// coefficient for coefficient, and no row can sum so many and so large terms
+// that rounding alone reaches the 1e-12 of the Hermiticity test (each side
+// adds the same numbers, in its own order). The operator then passes that
+// test without expanding its rows. False says nothing.
+bool hermitian_by_terms(const std::vector<Instance>& adjoint, const std::vector<Instance>& forward,
+                        const LocalFactors& f, int sites);
+
 // kLookupTableGeneric: the image table with the general tile kernel even
 // where the nearest-neighbour hop kernel applies (kept for comparisons).
 enum LookupMode : int { kLookupAuto = 0, kLookupTable = 1, kLookupSearch = 2, kLookupLegacy = 3,

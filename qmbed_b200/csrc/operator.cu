@@ -332,7 +332,9 @@ __device__ inline void dict_insert(unsigned long long* keys, double value, int* 
   const unsigned long long key = value_key(value);
   unsigned h = dict_hash(key) & (kDictSlots - 1);
   for (int probe = 0; probe < kDictSlots; ++probe) {
-    const unsigned long long prev = atomicCAS(keys + h, kDictEmpty, key);
+    // almost every value is there already: only an empty slot takes the atomic
+    unsigned long long prev = *reinterpret_cast<volatile unsigned long long*>(keys + h);
+    if (prev == kDictEmpty) prev = atomicCAS(keys + h, kDictEmpty, key);
     if (prev == kDictEmpty || prev == key) return;
     h = (h + 1) & (kDictSlots - 1);
   }
@@ -752,10 +754,9 @@ __global__ void __launch_bounds__(128) spmm_matrix_free_kernel(OpView<S> v, cons
   }
 }
 
-// Shapes of the block action tried by the autotuner: (ES, KB).
-constexpr int kBlockShapes = 4;
-constexpr int kBlockShapeES[kBlockShapes] = {1, 1, 2, 4};
-constexpr int kBlockShapeKB[kBlockShapes] = {4, 8, 4, 2};
+// Shapes of the block action tried by the autotuner: entry split and batch
+// of row lists (launch_block), block size and batch of tiled rows.
+constexpr int kBlockShapes = kTileBlockShapes;
 constexpr uint64_t kTuneMinRows = 1u << 20;  // smaller operators use shape 0 untimed
 
 // xs = x / sqrt(R) elementwise (complex vectors scale both parts).
@@ -884,7 +885,7 @@ SpinOperator::SpinOperator(std::shared_ptr<SpinBasis> basis, const std::vector<T
   inv_sqrt_.allocate(table.size() * sizeof(double));
   QMBED_CUDA(cudaMemcpy(inv_sqrt_.get(), table.data(), table.size() * sizeof(double), cudaMemcpyHostToDevice));
   // flip chains have real coefficients on symmetric flips and a real diagonal: Hermitian by construction
-  if (checks.hermiticity && !flip_ && !check_hermitian()) raise(QMBED_NON_HERMITIAN, "");
+  if (checks.hermiticity && !flip_ && !hermitian_terms_ && !check_hermitian()) raise(QMBED_NON_HERMITIAN, "");
   if (storage_ != kStorageMatrixFree) {
     if (dim() >= (1ULL << 32)) {
       storage_ = kStorageMatrixFree;  // columns do not fit 32 bits: keep the action matrix-free
@@ -892,6 +893,7 @@ SpinOperator::SpinOperator(std::shared_ptr<SpinBasis> basis, const std::vector<T
       assemble();
     }
   }
+  host_prog_.reset();
   // Matrix-free operators on a symmetry sector resolve their targets through
   // the basis's image table when it fits (built once, shared by every
   // operator on the basis); otherwise through the representative search.
@@ -1085,7 +1087,11 @@ void SpinOperator::build_instances(const std::vector<TermDesc>& terms, const Ope
       nnz_off_ = flips * dim();
     }
   }
-  if (basis_->words() == 1) prog_.upload(compile_flip_program(adj, factors_, sites, basis_->params().up >= 0));
+  if (basis_->words() == 1) {
+    host_prog_ = std::make_unique<FlipProgram>(compile_flip_program(adj, factors_, sites, basis_->params().up >= 0));
+    prog_.upload(*host_prog_);
+    hermitian_terms_ = checks.hermiticity && hermitian_by_terms(adj, fwd, factors_, sites);
+  }
   inst_adj_.allocate(std::max<size_t>(adj.size(), 1) * sizeof(Instance));
   inst_fwd_.allocate(std::max<size_t>(fwd.size(), 1) * sizeof(Instance));
   if (!adj.empty()) {
@@ -1114,7 +1120,48 @@ bool SpinOperator::check_hermitian() const {
   return (h & kFlagNonHermitian) == 0;
 }
 
+SpinOperator::SpinOperator(const SpinOperator& other, RowListTag)
+    : basis_(other.basis_), storage_(kStoragePacked), real_(other.real_), factors_(other.factors_),
+      n_inst_(other.n_inst_) {
+  auto copy = [](const DeviceBuffer& from, DeviceBuffer& to) {
+    to.allocate(std::max<size_t>(from.bytes(), 1));
+    QMBED_CUDA(cudaMemcpy(to.get(), from.get(), from.bytes(), cudaMemcpyDeviceToDevice));
+  };
+  copy(other.inst_adj_, inst_adj_);
+  copy(other.inst_fwd_, inst_fwd_);
+  copy(other.inv_sqrt_, inv_sqrt_);
+  assemble_row_lists();
+}
+
+const SpinOperator& SpinOperator::row_lists() const {
+  if (!tile_) return *this;
+  std::lock_guard<std::mutex> lock(row_lists_mu_);
+  QMBED_CUDA(cudaSetDevice(basis_->device()));
+  if (!row_lists_) row_lists_.reset(new SpinOperator(*this, RowListTag{}));
+  return *row_lists_;
+}
+
+// Rows in tiles of 32 where the operator has that form (one expansion, no
+// scaled input vector, coded complex values), else row lists.
 void SpinOperator::assemble() {
+  auto start = std::chrono::steady_clock::now();
+  if (storage_ == kStoragePacked && host_prog_) {
+    auto rows = std::make_unique<TileRows>();
+    if (assemble_tile_rows(*basis_, *host_prog_, real_, *rows)) {
+      nnz_off_ = rows->nnz;
+      col_bits_ = rows->col_bits;
+      // complex values were always counted as explicit ones
+      storage_ = real_ ? kStoragePacked : kStorageWide;
+      n_codes_ = real_ ? std::max(rows->distinct_values, 1) : 0;
+      tile_ = std::move(rows);
+      assembly_seconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
+      return;
+    }
+  }
+  assemble_row_lists();
+}
+
+void SpinOperator::assemble_row_lists() {
   auto start = std::chrono::steady_clock::now();
   const uint64_t n = dim();
   const int device_grid = grid_for(n, 128, 16);
@@ -1283,6 +1330,10 @@ void SpinOperator::apply(int precision, bool complex_vectors, const void* x, voi
     return;
   }
   // Stored rows.
+  if (tile_) {
+    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, x, y, stream);
+    return;
+  }
   const bool scaled = basis_->symmetric();
   const void* xs = x;
   if (scaled) {
@@ -1375,6 +1426,10 @@ void SpinOperator::apply_with_scratch(int precision, bool complex_vectors, const
     raise(QMBED_DIMENSION_MISMATCH, "symmetry sectors with stored rows take vectors of at most " +
                                         std::to_string(scratch_bytes) + " bytes here; this one has " +
                                         std::to_string(need));
+  if (tile_) {  // needs no scaled vector
+    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, x, y, stream);
+    return;
+  }
   {
     const int grid = grid_for(n * comps, 256, 16);
     if (precision == kFP64)
@@ -1425,6 +1480,7 @@ void SpinOperator::apply_with_scratch(int precision, bool complex_vectors, const
 
 SpinOperator::ExplicitRows SpinOperator::explicit_rows() const {
   if (storage_ != kStorageWide) raise(QMBED_UNSUPPORTED_BACKEND, "the operator does not hold rows with explicit values");
+  if (tile_) return row_lists().explicit_rows();
   ExplicitRows r;
   r.n = dim();
   r.row_ptr64 = row_ptr64_;
@@ -1484,6 +1540,10 @@ void SpinOperator::launch_block_matrix_free(int precision, int nb, const void* z
 
 void SpinOperator::launch_block(int shape, int precision, int nb, const void* z, const void* p, void* out,
                                 double alpha, double beta, double gamma, cudaStream_t stream) const {
+  if (tile_) {
+    tile_spmm(*tile_, shape, precision, nb, z, p, out, alpha, beta, gamma, stream);
+    return;
+  }
   const uint64_t n = dim();
   auto launch = [&](auto ttag, auto itag, auto nbtag, auto ptag, auto estag, auto kbtag) {
     using T = decltype(ttag);
@@ -1559,8 +1619,8 @@ int SpinOperator::block_shape(int precision, int nb, const void* z, const void* 
       }
       const char* trace = std::getenv("QMBED_FILTER_TRACE");
       if (trace && trace[0] == '1')
-        std::fprintf(stderr, "[block tune] fp%d nb=%d p=%d shape ES=%d KB=%d: %.3f ms\n", precision, nb, p ? 1 : 0,
-                     kBlockShapeES[shape], kBlockShapeKB[shape], ms / 3.0f);
+        std::fprintf(stderr, "[block tune] fp%d nb=%d p=%d shape %d: %.3f ms\n", precision, nb, p ? 1 : 0, shape,
+                     ms / 3.0f);
     }
     cudaEventDestroy(start);
     cudaEventDestroy(stop);
@@ -1614,6 +1674,10 @@ void SpinOperator::export_csr(std::vector<uint64_t>& row_ptr, std::vector<uint32
                               std::vector<C64>& values) const {
   QMBED_CUDA(cudaSetDevice(basis_->device()));
   if (storage_ == kStorageMatrixFree) raise(QMBED_UNSUPPORTED_BACKEND, "matrix-free operators hold no stored rows");
+  if (tile_) {
+    row_lists().export_csr(row_ptr, cols, values);
+    return;
+  }
   const uint64_t n = dim();
   row_ptr.resize(n + 1);
   if (row_ptr64_) {

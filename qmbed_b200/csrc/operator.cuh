@@ -12,6 +12,7 @@
 #include "basis.cuh"
 #include "flipchain.cuh"
 #include "hv_tile.cuh"
+#include "tile_rows.cuh"
 
 namespace qmbed {
 
@@ -158,8 +159,14 @@ class SpinOperator {
   bool chain_form() const { return prog_.ok() && prog_.chain_ok(); }
 
  private:
+  struct RowListTag {};
+  // The same operator with its rows as row lists, whatever its own storage.
+  SpinOperator(const SpinOperator& other, RowListTag);
+  const SpinOperator& row_lists() const;
+
   void build_instances(const std::vector<TermDesc>& terms, const OperatorChecks& checks);
   void assemble();
+  void assemble_row_lists();
   void ensure_scratch(int precision, bool complex_vectors) const;
   void launch_block_matrix_free(int precision, int nb, const void* z, const void* p, void* out, double alpha,
                                 double beta, double gamma, cudaStream_t stream) const;
@@ -175,7 +182,13 @@ class SpinOperator {
   int n_inst_ = 0;
   DeviceBuffer inst_adj_, inst_fwd_;
   DeviceBuffer inv_sqrt_;   // 257 doubles: 1/sqrt(R)
-  // Assembled storage.
+  // Assembled storage: rows in tiles when the operator has that form, else row
+  // lists (columns with value codes, or with explicit values).
+  std::unique_ptr<TileRows> tile_;
+  mutable std::unique_ptr<SpinOperator> row_lists_;  // of a tiled operator, on first use
+  mutable std::mutex row_lists_mu_;
+  std::unique_ptr<FlipProgram> host_prog_;  // until the rows are assembled
+  bool hermitian_terms_ = false;            // Hermitian by its products alone
   uint64_t nnz_off_ = 0;
   int col_bits_ = 0, n_codes_ = 0;
   bool row_ptr64_ = false;
