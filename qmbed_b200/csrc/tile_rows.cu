@@ -385,8 +385,19 @@ __device__ __forceinline__ typename Pair2<T>::type load_complex(const T* x, uint
 // y[r] = sqrt(R_r) sum_e value[code_e] x[col_e] + d[r] x[r], one lane per row.
 // VC: complex vectors; VALC: complex values. With SPLIT > 1 a block of SPLIT
 // warps shares one tile's slots (small sectors), else every warp has a tile of its own.
+//
+// Bound by the gathers' way through the L2: a slot of 32 rows touches 15 (FP64)
+// or 11 (FP32) sectors of 32, and DRAM carries little more than the entries
+// (x stays in the L2). Small blocks and few registers win, because the rows'
+// latency chain (tile pointer, entries, gathers) is hidden by warps in flight:
+// blocks of 128 threads against 1024 were 20.8 against 24.2 us at 28 sites
+// (718,146 rows, FP64) and 119 against 145 us at 31 (4,850,640 rows). Against
+// row lists with a scaled copy of x (measured in the same call): 34.7 -> 20.8
+// us and 212 -> 119 us; complex rows of 26 sites at k = 3 (400,023 rows, 20
+// bytes per entry before, 4 now) 85.5 -> 40 us.
+constexpr int kSpmvThreads = 128;
 template <typename T, bool VC, bool VALC, bool VEC2, int SPLIT, int KB>
-__global__ void __launch_bounds__(1024) tile_spmv_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
+__global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
                                                          const uint32_t* __restrict__ entries, int col_bits,
                                                          const double2* __restrict__ values, int codes,
                                                          const T* __restrict__ diag,
@@ -397,27 +408,29 @@ __global__ void __launch_bounds__(1024) tile_spmv_kernel(uint64_t n, const uint3
   using V = typename std::conditional<VALC, P, T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   V* table = reinterpret_cast<V*>(smem);
-  for (int i = threadIdx.x; i < codes; i += blockDim.x) {
-    const double2 v = values[i];
-    if constexpr (VALC) {
-      table[i].x = static_cast<T>(v.x);
-      table[i].y = static_cast<T>(v.y);
-    } else {
-      table[i] = static_cast<T>(v.x);
-    }
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t tiles = (n + 31) / 32;
   const uint64_t t = SPLIT > 1 ? blockIdx.x : static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
   const uint32_t col_mask = (1u << col_bits) - 1u;
-  T ar = 0, ai = 0;
   const uint64_t r = t * 32 + lane;
   const bool valid = t < tiles && r < n;
+  int from = 0, to = 0;
+  const uint32_t* row = entries + lane;
+  uint32_t e[KB];
+  if (t < tiles) {
+    const uint32_t base = __ldg(tile_ptr + t);
+    const int width = static_cast<int>(__ldg(tile_ptr + t + 1) - base);
+    from = SPLIT > 1 ? width * warp / SPLIT : 0;
+    to = SPLIT > 1 ? width * (warp + 1) / SPLIT : width;
+    row += static_cast<uint64_t>(base) * 32;
+  }
+  // the first entries and the row's own operands are requested before the
+  // code table is staged, the next entries before the current ones are used
+#pragma unroll
+  for (int u = 0; u < KB; ++u) e[u] = from + u < to ? load_entry(row + (from + u) * 32) : kNoEntry;
   T xr = 0, xi = 0, dr = 0, di = 0;
   uint32_t orbit = 0;
   if (valid && (SPLIT == 1 || warp == 0)) {
-    // requested before the entries so that their latency overlaps the row
     if (VC) {
       const P v = load_complex<T, VEC2>(x, r);
       xr = v.x;
@@ -433,32 +446,37 @@ __global__ void __launch_bounds__(1024) tile_spmv_kernel(uint64_t n, const uint3
     }
     if (orbits) orbit = __ldcs(orbits + r);
   }
-  if (t < tiles) {
-    const uint32_t base = __ldg(tile_ptr + t);
-    const int width = static_cast<int>(__ldg(tile_ptr + t + 1) - base);
-    const int from = SPLIT > 1 ? width * warp / SPLIT : 0;
-    const int to = SPLIT > 1 ? width * (warp + 1) / SPLIT : width;
-    const uint32_t* row = entries + static_cast<uint64_t>(base) * 32 + lane;
-    for (int j0 = from; j0 < to; j0 += KB) {
-      uint32_t e[KB];
+  for (int i = threadIdx.x; i < codes; i += blockDim.x) {
+    const double2 v = values[i];
+    if constexpr (VALC) {
+      table[i].x = static_cast<T>(v.x);
+      table[i].y = static_cast<T>(v.y);
+    } else {
+      table[i] = static_cast<T>(v.x);
+    }
+  }
+  __syncthreads();
+  T ar = 0, ai = 0;
+  for (int j0 = from; j0 < to; j0 += KB) {
+    T gr[KB], gi[KB];
 #pragma unroll
-      for (int u = 0; u < KB; ++u) e[u] = j0 + u < to ? load_entry(row + (j0 + u) * 32) : kNoEntry;
-      T gr[KB], gi[KB];
-#pragma unroll
-      for (int u = 0; u < KB; ++u) {
-        gr[u] = gi[u] = 0;
-        if (e[u] == kNoEntry) continue;
-        if (VC) {
-          const P v = load_complex<T, VEC2>(x, e[u] & col_mask);
-          gr[u] = v.x;
-          gi[u] = v.y;
-        } else {
-          gr[u] = __ldg(x + (e[u] & col_mask));
-        }
+    for (int u = 0; u < KB; ++u) {
+      gr[u] = gi[u] = 0;
+      if (e[u] == kNoEntry) continue;
+      if (VC) {
+        const P v = load_complex<T, VEC2>(x, e[u] & col_mask);
+        gr[u] = v.x;
+        gi[u] = v.y;
+      } else {
+        gr[u] = __ldg(x + (e[u] & col_mask));
       }
+    }
+    uint32_t f[KB];
 #pragma unroll
-      for (int u = 0; u < KB; ++u) {
-        if (e[u] == kNoEntry) continue;
+    for (int u = 0; u < KB; ++u) f[u] = j0 + KB + u < to ? load_entry(row + (j0 + KB + u) * 32) : kNoEntry;
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      if (e[u] != kNoEntry) {
         const V c = table[e[u] >> col_bits];
         if constexpr (VALC) {
           ar += c.x * gr[u] - c.y * gi[u];
@@ -468,6 +486,7 @@ __global__ void __launch_bounds__(1024) tile_spmv_kernel(uint64_t n, const uint3
           if (VC) ai += c * gi[u];
         }
       }
+      e[u] = f[u];
     }
   }
   if (SPLIT > 1) {
@@ -507,9 +526,12 @@ __global__ void __launch_bounds__(1024) tile_spmv_kernel(uint64_t n, const uint3
 // Block action on tiles: a row's NB values are LPR consecutive 16-byte
 // vectors, one per lane, and a warp takes 32 / LPR rows of a tile (LPR
 // neighbouring warps share one). Entries are read once per row and shared by
-// its lanes.
+// its lanes. Bound by the L2: every gathered column is 32 to 128 bytes, and at
+// 32 sites (9,398,520 rows, FP32, 8 columns) the 634 us move 6.6 GB through it
+// (10.4 TB/s); the row lists took 766 us. At 28 sites (718,146 rows, 16
+// columns) 70 against 75 us in FP32 and 138 against 139 us in FP64.
 template <typename T, int NB, bool HAS_P, int KB>
-__global__ void __launch_bounds__(1024) tile_spmm_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
+__global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
                                                          const uint32_t* __restrict__ entries, int col_bits,
                                                          const double2* __restrict__ values, int codes,
                                                          const T* __restrict__ diag, const T* __restrict__ z,
@@ -519,25 +541,29 @@ __global__ void __launch_bounds__(1024) tile_spmm_kernel(uint64_t n, const uint3
   constexpr int RPW = 32 / LPR;
   extern __shared__ __align__(16) unsigned char smem[];
   T* table = reinterpret_cast<T*>(smem);
-  for (int i = threadIdx.x; i < codes; i += blockDim.x) table[i] = static_cast<T>(values[i].x);
-  __syncthreads();
   const int lane = threadIdx.x & 31;
   const uint64_t w = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const uint64_t t = w / LPR;
   const int in_tile = static_cast<int>(w % LPR) * RPW + lane / LPR, part = lane % LPR;
   const uint64_t r = t * 32 + in_tile;
-  if (r >= n) return;
   const uint32_t col_mask = (1u << col_bits) - 1u;
-  const uint32_t base = __ldg(tile_ptr + t);
-  const int width = static_cast<int>(__ldg(tile_ptr + t + 1) - base);
-  const uint32_t* row = entries + static_cast<uint64_t>(base) * 32 + in_tile;
+  int width = 0;
+  const uint32_t* row = entries + in_tile;
+  uint32_t e[KB];
+  if (r < n) {
+    const uint32_t base = __ldg(tile_ptr + t);
+    width = static_cast<int>(__ldg(tile_ptr + t + 1) - base);
+    row += static_cast<uint64_t>(base) * 32;
+  }
+#pragma unroll
+  for (int u = 0; u < KB; ++u) e[u] = u < width ? __ldg(row + u * 32) : kNoEntry;
+  for (int i = threadIdx.x; i < codes; i += blockDim.x) table[i] = static_cast<T>(values[i].x);
+  __syncthreads();
+  if (r >= n) return;
   T acc[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) acc[v] = 0;
   for (int j0 = 0; j0 < width; j0 += KB) {
-    uint32_t e[KB];
-#pragma unroll
-    for (int u = 0; u < KB; ++u) e[u] = j0 + u < width ? __ldg(row + (j0 + u) * 32) : kNoEntry;
     T g[KB][VEC];
 #pragma unroll
     for (int u = 0; u < KB; ++u) {
@@ -554,6 +580,8 @@ __global__ void __launch_bounds__(1024) tile_spmm_kernel(uint64_t n, const uint3
 #pragma unroll
       for (int v = 0; v < VEC; ++v) acc[v] += c * g[u][v];
     }
+#pragma unroll
+    for (int u = 0; u < KB; ++u) e[u] = j0 + KB + u < width ? __ldg(row + (j0 + KB + u) * 32) : kNoEntry;
   }
   const T d = __ldcs(diag + r);
   T self[VEC], o[VEC];
@@ -799,9 +827,16 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
 
 namespace {
 
-// Sectors below this many tiles take four warps per tile: one warp per tile
-// would leave most of the SMs' warp slots empty and a row's gathers in series.
-constexpr uint64_t kSplitTiles = 148 * 16;
+// Sectors below this many tiles take four warps per tile: with one warp each,
+// fewer than eight warps would sit on an SM and a row's gathers run in series
+// (complex rows of 22 sites, 1003 tiles: 6.8 against 8.4 us a call; at 1776
+// tiles, 24 sites, 7.2 against 6.8).
+constexpr uint64_t kSplitTiles = 148 * 8;
+// Real FP64 rows keep eight gathers in flight per lane from here on: at 28
+// sites (718,146 rows) four take 20.8 us and eight 21.8, at 30 (2,587,018) 75.0
+// and 70.3, at 31 131.5 and 119.2. In FP32 and with complex vectors four are
+// faster at every size (32 sites FP32 187 against 212 us).
+constexpr uint64_t kDeepRows = 1ull << 21;
 
 template <typename T, bool VC, bool VALC, bool VEC2>
 void launch_spmv(const TileRows& rows, const SpinBasis& basis, const double* sqrt_table, const T* diag, const void* x,
@@ -810,18 +845,17 @@ void launch_spmv(const TileRows& rows, const SpinBasis& basis, const double* sqr
   const size_t smem = static_cast<size_t>(rows.codes) * sizeof(T) * (VALC ? 2 : 1);
   const double2* values = rows.values.as<double2>() + rows.codes;
   const uint16_t* orbits = basis.symmetric() ? basis.orbits() : nullptr;
-  constexpr int KB = VC && sizeof(T) == 8 ? 4 : 8;
-  if (tiles <= kSplitTiles) {
-    tile_spmv_kernel<T, VC, VALC, VEC2, 4, 4><<<static_cast<unsigned>(tiles), 128, smem, stream>>>(
+  auto launch = [&](auto kernel, uint64_t blocks) {
+    kernel<<<static_cast<unsigned>(blocks), kSpmvThreads, smem, stream>>>(
         rows.n, rows.tile_ptr.as<uint32_t>(), rows.entries.as<uint32_t>(), rows.col_bits, values, rows.codes, diag,
         orbits, sqrt_table, static_cast<const T*>(x), static_cast<T*>(y));
-  } else {
-    const int threads = 1024;
-    const unsigned grid = static_cast<unsigned>((tiles + threads / 32 - 1) / (threads / 32));
-    tile_spmv_kernel<T, VC, VALC, VEC2, 1, KB><<<grid, threads, smem, stream>>>(
-        rows.n, rows.tile_ptr.as<uint32_t>(), rows.entries.as<uint32_t>(), rows.col_bits, values, rows.codes, diag,
-        orbits, sqrt_table, static_cast<const T*>(x), static_cast<T*>(y));
-  }
+  };
+  constexpr int kWarps = kSpmvThreads / 32;
+  const uint64_t blocks = (tiles + kWarps - 1) / kWarps;
+  constexpr int kDeep = !VC && sizeof(T) == 8 ? 8 : 4;
+  if (tiles <= kSplitTiles) launch(tile_spmv_kernel<T, VC, VALC, VEC2, kWarps, 4>, tiles);
+  else if (rows.n >= kDeepRows) launch(tile_spmv_kernel<T, VC, VALC, VEC2, 1, kDeep>, blocks);
+  else launch(tile_spmv_kernel<T, VC, VALC, VEC2, 1, 4>, blocks);
   QMBED_LAUNCH_CHECK();
 }
 
@@ -852,8 +886,8 @@ void tile_spmv(const TileRows& rows, const SpinBasis& basis, const double* sqrt_
 void tile_spmm(const TileRows& rows, int shape, int precision, int nb, const void* z, const void* p, void* out,
                double alpha, double beta, double gamma, cudaStream_t stream) {
   const uint64_t tiles = (rows.n + 31) / 32;
-  static constexpr int kThreadsOf[kTileBlockShapes] = {256, 256, 512, 1024};
-  static constexpr bool kDeep[kTileBlockShapes] = {false, true, false, false};
+  static constexpr int kThreadsOf[kTileBlockShapes] = {64, 128, 64, 256};
+  static constexpr int kBatchOf[kTileBlockShapes] = {4, 4, 2, 8};
   auto launch = [&](auto ttag, auto nbtag, auto ptag, auto kbtag) {
     using T = decltype(ttag);
     constexpr int NB = decltype(nbtag)::value;
@@ -871,7 +905,8 @@ void tile_spmm(const TileRows& rows, int shape, int precision, int nb, const voi
             static_cast<T*>(out), static_cast<T>(alpha), static_cast<T>(beta), static_cast<T>(gamma));
   };
   auto by_kb = [&](auto ttag, auto nbtag, auto ptag) {
-    if (kDeep[shape]) launch(ttag, nbtag, ptag, std::integral_constant<int, 8>{});
+    if (kBatchOf[shape] == 8) launch(ttag, nbtag, ptag, std::integral_constant<int, 8>{});
+    else if (kBatchOf[shape] == 2) launch(ttag, nbtag, ptag, std::integral_constant<int, 2>{});
     else launch(ttag, nbtag, ptag, std::integral_constant<int, 4>{});
   };
   auto by_p = [&](auto ttag, auto nbtag) {
