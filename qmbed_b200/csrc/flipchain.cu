@@ -1,16 +1,13 @@
 // Structured full-space chain action (diagonal z products + single bit flips).
 //
-// The action is y[s] = D(s) x[s] + sum_i c_i x[s ^ (1 << i)], computed in one
-// pass over tiles of 2^tb consecutive elements (64 KB) held in shared memory:
-// the flips of the low tb bits read the tile, the flips of the higher bits
-// read their partner element from global memory. A partner of bit i lies in
-// tile t ^ 2^(i - tb), a contiguous chunk, so those reads are fully coalesced,
-// and partner tiles within the L2 window (about 1900 tiles of 64 KB) are
-// served by L2. The fused epilogue out = alpha y + beta x + gamma p + kappa q
-// serves the Chebyshev (Clenshaw) step.
-// D(s) = D_low(j) + D_high(t) + D_cross(s): terms inside the low bits come from
-// a 2^tb table computed once, terms inside the high bits once per tile, and
-// only the terms spanning both are evaluated per element.
+// The action is y[s] = D(s) x[s] + sum_i c_i x[s ^ (1 << i)], with the fused
+// epilogue out = alpha y + beta x + gamma p + kappa q of the Chebyshev
+// (Clenshaw) step. Vectors move through boxes of 16-byte words in shared
+// memory: the flips inside a box read the box (or the thread's own
+// registers), the other flips read their partner from global memory, or take
+// a pass of their own over boxes that span those bits (flip_box_kernel).
+// Chains too short for a box, vectors that start off a 16-byte boundary and
+// calls that write over x or q take flip_chain_kernel, one tile per block.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -103,9 +100,8 @@ __global__ void diag_low_table_kernel(int tb, int nd, const uint64_t* __restrict
 }
 
 // D_high[t] = sum over terms with mask inside the bits >= tb of c (-1)^popcount(~(t << tb) & mask)
-template <typename T>
 __global__ void diag_high_table_kernel(int tb, int sites, int nd, const uint64_t* __restrict__ masks,
-                                       const double* __restrict__ coefs, T* __restrict__ table) {
+                                       const double* __restrict__ coefs, double* __restrict__ table) {
   const uint64_t low = (1ull << tb) - 1ull;
   const uint64_t count = 1ull << (sites - tb);
   for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < count;
@@ -114,11 +110,15 @@ __global__ void diag_high_table_kernel(int tb, int sites, int nd, const uint64_t
     double d = 0.0;
     for (int k = 0; k < nd; ++k)
       if (masks[k] != 0 && (masks[k] & low) == 0) d += (__popcll(~base & masks[k]) & 1) ? -coefs[k] : coefs[k];
-    table[t] = static_cast<T>(d);
+    table[t] = d;
   }
 }
 
-// One pass: tile flips, global-partner flips, diagonal and the epilogue.
+// One pass over tiles of 2^tb consecutive elements (64 KB): flips of the low tb
+// bits read the tile, flips of the higher bits their partner element in global memory.
+// D(s) = D_low(j) + D_high(t) + D_cross(s): terms inside the low bits come from
+// a 2^tb table computed once, terms inside the high bits once per tile, and
+// only the terms spanning both are evaluated per element.
 // TB > 0 fixes the tile bits at compile time (the tile loop unrolls); TB = 0
 // takes them from `tb` (chains shorter than a tile).
 template <typename T, bool CPLX, int TB>
@@ -202,24 +202,36 @@ int log2_int(int v) {
 }
 
 // ---------------------------------------------------------------------------
-// Multi-pass action for chains whose vectors exceed the L2 (TMA-staged boxes)
+// Box action (TMA-staged boxes)
 // ---------------------------------------------------------------------------
 //
-// Pass A applies the diagonal and the flips of the low TB bits to contiguous
-// boxes of 2^TB elements and writes the whole epilogue
-//   out = alpha (D x + sum_{i < TB} c_i x[s ^ 2^i]) + beta x + gamma p + kappa q.
-// Each later pass takes a group of G higher bits [b0, b0 + G): a box holds the
-// 2^G elements that differ only in those bits, for a 64-byte run of the lowest
-// bits and a batch of the bits above the run, so every flip of the group is a
-// read of the box in shared memory; it adds alpha sum_{i in group} c_i x[s ^ 2^i]
-// to out. Boxes come in by TMA (cp.async.bulk for pass A, cp.async.bulk.tensor
-// for the strided group boxes) into two shared-memory stages, so the next box
-// loads while the current one is used. Every wait on a stage's mbarrier is
-// bounded: on time-out the block records the failure in `status` and stops.
+// A box holds 2^VB words of 16 bytes in shared memory. The first launch takes
+// contiguous boxes (cp.async.bulk): diagonal, the flips of the bits inside the
+// word and the box, the flips of `extra` bits above the box by direct reads of
+// the partner words, and the whole epilogue. For vectors far beyond the L2 a
+// group pass takes the top bits [b0, b0 + G): its box (cp.async.bulk.tensor) is
+// a 64-byte run, a batch of the bits above the run and all values of the
+// group's bits, so every flip of the group stays inside the box; it adds
+// alpha sum c_i x[s ^ 2^i] to out.
+//
+// What bounds it: every flip of a word costs one 16-byte read per thread,
+// from shared memory or from the L2, except those between words that one
+// thread owns, so the load pipe is the limit (21 reads and writes per word at
+// 22 sites; 62% of its rate) and the L2 serves the direct reads at 13 TB/s. A
+// thread owns eight words that differ in the top three bits of the box; each
+// serves its diagonal and the flips along those bits as it is read, and is not
+// kept, so that many small boxes (16 KB, 128 threads) stay resident. Larger
+// boxes with fewer direct reads were slower (64 KB boxes with a group pass at
+// 22 sites in complex128: 86 us), persistent blocks with a box pipeline slower
+// still (109 us). Measured against the earlier kernels (64 KB tiles with one
+// element per thread and step; three passes from 256 MB on): complex128 H.v of
+// 22 sites 105 -> 63 to 72 us, 24 sites 440 -> 280 us, complex64 of 24 sites
+// 284 -> 122 us, 25 sites 522 -> 286 us, 28 sites 4.1 -> 2.7 ms; with p and q
+// 125 -> 84 us at 22 sites in complex128.
 
-constexpr int kPassThreads = 512;
-constexpr int kBoxBytes = 32 * 1024;
-constexpr int kStages = 3;
+constexpr int kBoxMaxWords = 12;  // word bits of a group pass's box (64 KB)
+constexpr int kBoxMaxExtra = 16;  // flips above the box by direct reads
+constexpr int kBoxLaneBits = 5;
 constexpr unsigned kWaitPolls = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -252,176 +264,369 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
-__device__ __forceinline__ void tensor_load5(void* dst, const CUtensorMap* map, int c1, int c4, uint64_t* bar) {
+__device__ __forceinline__ void tensor_load5(void* dst, const CUtensorMap* map, int c1, int c3, int c4, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
       "%6}], [%7];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(0), "r"(0), "r"(c4), "r"(smem_addr(bar))
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(0), "r"(c3), "r"(c4), "r"(smem_addr(bar))
       : "memory");
 }
 
-// One pass of the multi-pass action. GROUP = false: pass A over contiguous
-// boxes; GROUP = true: the group [b0, b0 + G) from tensor-map boxes.
-struct PassArgs {
-  int sites, b0, G, bb;  // group pass: box = run (R bits) x batch (bb bits) x group (G bits)
-  int nd;
-  const uint64_t* masks;
-  const double* coefs;
-  const void* low_table;
-  const void* high_table;  // pass A: the diagonal part of the bits above the box, per box
-  const double* xcoef;
-  const void* x;
-  void* out;
-  const void* p;
-  const void* q;
-  double alpha, beta, gamma, kr, ki;
+// A 16-byte word as the kernels compute on it: four floats (two packed pairs)
+// or two doubles.
+template <typename T>
+struct Word;
+template <>
+struct Word<float> {
+  unsigned long long a, b;
+};
+template <>
+struct Word<double> {
+  double a, b;
+};
+template <typename T>
+struct Coef;  // a real factor in the form axpy() takes
+template <>
+struct Coef<float> {
+  using type = unsigned long long;
+};
+template <>
+struct Coef<double> {
+  using type = double;
+};
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long x, unsigned long long y, unsigned long long z) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  return r;
+}
+__device__ __forceinline__ unsigned long long coef_of(float c) { return pack2(c, c); }
+__device__ __forceinline__ double coef_of(double c) { return c; }
+__device__ __forceinline__ void axpy(Word<float>& acc, unsigned long long c, const Word<float>& v) {
+  acc.a = fma2(c, v.a, acc.a);
+  acc.b = fma2(c, v.b, acc.b);
+}
+__device__ __forceinline__ void axpy(Word<double>& acc, double c, const Word<double>& v) {
+  acc.a = fma(c, v.a, acc.a);
+  acc.b = fma(c, v.b, acc.b);
+}
+__device__ __forceinline__ Word<float> load_word(const Word<float>* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return Word<float>{v.x, v.y};
+}
+__device__ __forceinline__ Word<double> load_word(const Word<double>* p) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  return Word<double>{v.x, v.y};
+}
+__device__ __forceinline__ void store_word(Word<float>* p, const Word<float>& v) {
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.a, v.b);
+}
+__device__ __forceinline__ void store_word(Word<double>* p, const Word<double>& v) {
+  *reinterpret_cast<double2*>(p) = make_double2(v.a, v.b);
+}
+
+// Element layout of a word: EV elements, VBITS = log2(EV) bits of the state
+// index inside it.
+template <typename T, bool CPLX>
+struct WordShape {
+  static constexpr int EV = 16 / (static_cast<int>(sizeof(T)) * (CPLX ? 2 : 1));
+  static constexpr int VBITS = EV == 1 ? 0 : (EV == 2 ? 1 : 2);
+};
+
+// acc += diag(m_0 .. m_EV-1) v, one factor per element
+template <bool CPLX>
+__device__ __forceinline__ void axpy_diag(Word<float>& acc, const float* m, const Word<float>& v) {
+  acc.a = fma2(CPLX ? pack2(m[0], m[0]) : pack2(m[0], m[1]), v.a, acc.a);
+  acc.b = fma2(CPLX ? pack2(m[1], m[1]) : pack2(m[2], m[3]), v.b, acc.b);
+}
+template <bool CPLX>
+__device__ __forceinline__ void axpy_diag(Word<double>& acc, const double* m, const Word<double>& v) {
+  acc.a = fma(m[0], v.a, acc.a);
+  acc.b = fma(CPLX ? m[0] : m[1], v.b, acc.b);
+}
+// the word with its elements exchanged along state bit `bit` < VBITS
+template <bool CPLX>
+__device__ __forceinline__ Word<float> flip_inside(const Word<float>& v, int bit) {
+  if (CPLX || bit == 1) return Word<float>{v.b, v.a};
+  const float2 x = unpack2(v.a), y = unpack2(v.b);
+  return Word<float>{pack2(x.y, x.x), pack2(y.y, y.x)};
+}
+template <bool CPLX>
+__device__ __forceinline__ Word<double> flip_inside(const Word<double>& v, int) {
+  return Word<double>{v.b, v.a};
+}
+// kappa q (real vectors: its real part)
+template <bool CPLX>
+__device__ __forceinline__ Word<float> kappa_word(float kr, float ki, const Word<float>& q) {
+  if (!CPLX) return Word<float>{fma2(pack2(kr, kr), q.a, 0ull), fma2(pack2(kr, kr), q.b, 0ull)};
+  const float2 x = unpack2(q.a), y = unpack2(q.b);
+  return Word<float>{pack2(kr * x.x - ki * x.y, kr * x.y + ki * x.x), pack2(kr * y.x - ki * y.y, kr * y.y + ki * y.x)};
+}
+template <bool CPLX>
+__device__ __forceinline__ Word<double> kappa_word(double kr, double ki, const Word<double>& q) {
+  if (!CPLX) return Word<double>{kr * q.a, kr * q.b};
+  return Word<double>{kr * q.a - ki * q.b, kr * q.b + ki * q.a};
+}
+
+template <typename T>
+struct BoxArgs {
+  using C = typename Coef<T>::type;
+  int sites;
+  int extra;      // flips above the box by direct reads
+  int b0, G, bb;  // group pass: bits [b0, b0 + G), bb batch bits above the 64-byte run
+  int lo;         // group pass: lowest word bit of the box with a flip
+  // alpha c of the flips, by value: the multiply-adds take them from constant memory
+  C cbit[kBoxMaxWords];    // along a word bit of the box
+  C cinside[2];            // inside the word
+  C cextra[kBoxMaxExtra];  // above the box
+  // Diagonal, split by the bits a term holds: inside the
+  // lanes' bits (lane_table, per lane and element), inside the other bits of
+  // the box (word_table), above the box (high_table, per box), spanning the
+  // lanes' bits and others (terms 0 .. n_lane - 1) and spanning the other box
+  // bits and those above (the next n_word terms).
+  // Tables and sums in FP64: alpha D + beta is rounded to T once.
+  const double* lane_table;
+  const double* word_table;
+  const double* high_table;
+  const uint64_t* span_masks;
+  const double* span_coefs;
+  int n_lane, n_word;
+  const Word<T>* x;
+  Word<T>* out;
+  const Word<T>* p;
+  const Word<T>* q;
+  double alpha, beta;
+  T gamma, kr, ki;
   int* status;
 };
 
-template <typename T, bool CPLX, int TB, int R, bool GROUP>
-__global__ void __launch_bounds__(kPassThreads, 2) flip_pass_kernel(const __grid_constant__ CUtensorMap map,
-                                                                 const PassArgs a) {
-  using E = typename Elem<T, CPLX>::type;
-  constexpr int kBox = 1 << TB;
-  constexpr int kPer = kBox / kPassThreads;
-  static_assert(kBox % kPassThreads == 0, "box elements must divide among the threads");
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  E* stage_buf = reinterpret_cast<E*>(smem_raw);
-  __shared__ __align__(8) uint64_t full[kStages];
-  __shared__ T cx[64];
-  __shared__ uint64_t cross_mask[kMaxDiagTerms];
-  __shared__ T cross_coef[kMaxDiagTerms];
-  __shared__ int n_cross;
-  __shared__ T d_high;
-  __shared__ int abort_flag;
-  __shared__ unsigned long long failed_box;
-  const int L = a.sites;
-  if (threadIdx.x < L) cx[threadIdx.x] = static_cast<T>(a.xcoef[threadIdx.x]);
-  const uint64_t low = (1ull << TB) - 1ull;
-  if (threadIdx.x == 0) {
-    int c = 0;
-    if (!GROUP)
-      for (int k = 0; k < a.nd; ++k)
-        if ((a.masks[k] & low) != 0 && (a.masks[k] & ~low) != 0) {
-          cross_mask[c] = a.masks[k];
-          cross_coef[c] = static_cast<T>(a.coefs[k]);
-          ++c;
-        }
-    n_cross = c;
-    abort_flag = 0;
-    for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+constexpr int kRegBits = 3;  // a thread's eight words differ in the top bits of the box
+constexpr int kWordsPerThread = 1 << kRegBits;
+
+// Loads that stay where they are written (before the wait on a box).
+__device__ __forceinline__ Word<float> load_early(const Word<float>* p) {
+  Word<float> v;
+  asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.a), "=l"(v.b) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ Word<double> load_early(const Word<double>* p) {
+  Word<double> v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.a), "=d"(v.b) : "l"(p));
+  return v;
+}
+
+// Diagonal of box `id` without the terms that touch the lanes' bits, for the
+// words u << kBoxLaneBits.
+template <typename T, int VB, int VBITS>
+__device__ __forceinline__ double word_diagonal(const BoxArgs<T>& a, uint64_t id, int u) {
+  const uint64_t s = (id << (VB + VBITS)) | (static_cast<uint64_t>(u) << (kBoxLaneBits + VBITS));
+  double d = a.word_table[u] + a.high_table[id];
+  for (int k = a.n_lane; k < a.n_lane + a.n_word; ++k) {
+    const double c = a.span_coefs[k];
+    d += (__popcll(~s & a.span_masks[k]) & 1) ? -c : c;
   }
+  return d;
+}
+
+// The diagonal of the thread's words v0 | j << LOW (word v of a box).
+template <typename T, bool CPLX, int VB>
+struct BoxDiagonal {
+  static constexpr int EV = WordShape<T, CPLX>::EV, VBITS = WordShape<T, CPLX>::VBITS;
+  double lane[EV];
+  uint64_t mask0 = 0;
+  double coef0 = 0.0;
+  __device__ __forceinline__ explicit BoxDiagonal(const BoxArgs<T>& a) {
+#pragma unroll
+    for (int e = 0; e < EV; ++e) lane[e] = __ldg(a.lane_table + (threadIdx.x & 31) * EV + e);
+    if (a.n_lane > 0) {
+      mask0 = __ldg(a.span_masks);
+      coef0 = __ldg(a.span_coefs);
+    }
+  }
+  // acc += (alpha D + beta) x of word v
+  __device__ __forceinline__ void add(const BoxArgs<T>& a, uint64_t gbase, const double* dword, int v,
+                                      const Word<T>& own, Word<T>& acc) const {
+    const uint64_t s = (gbase | static_cast<uint64_t>(v)) << VBITS;
+    const double du = dword[v >> kBoxLaneBits];
+    double m[EV];
+#pragma unroll
+    for (int e = 0; e < EV; ++e) m[e] = lane[e] + du + ((__popcll(~(s | e) & mask0) & 1) ? -coef0 : coef0);
+    for (int k = 1; k < a.n_lane; ++k) {
+      const uint64_t mask = __ldg(a.span_masks + k);
+      const double c = __ldg(a.span_coefs + k);
+#pragma unroll
+      for (int e = 0; e < EV; ++e) m[e] += (__popcll(~(s | e) & mask) & 1) ? -c : c;
+    }
+    T factor[EV];
+#pragma unroll
+    for (int e = 0; e < EV; ++e) factor[e] = static_cast<T>(a.alpha * m[e] + a.beta);
+    axpy_diag<CPLX>(acc, factor, own);
+  }
+};
+
+// Flips of the thread's words v0 | j << LOW, one eighth of the box after the
+// other: wait(j) is called before the j-th eighth is read. A word gives the
+// flips of its own bits to its sum (and whatever `own` adds), the flips along
+// the register bits to the sums of the seven other eighths, and takes the
+// flips along the lower bits from partners in its own eighth. So arithmetic
+// starts with the first eighth that arrives, and sum j is complete after
+// eighth max(j, j ^ 4). GROUP: only the flips along word bits >= a.lo.
+template <typename T, bool CPLX, int VB, bool GROUP, typename Wait, typename Own>
+__device__ __forceinline__ bool box_flips(const BoxArgs<T>& a, const Word<T>* box, int v0, Wait&& wait, Own&& own_part,
+                                          Word<T> (&acc)[kWordsPerThread]) {
+  constexpr int VBITS = WordShape<T, CPLX>::VBITS;
+  constexpr int LOW = VB - kRegBits;
+#pragma unroll
+  for (int j = 0; j < kWordsPerThread; ++j) {
+    if (!wait(j)) return false;
+    const int v = v0 | (j << LOW);
+    const Word<T> own = load_word(box + v);
+    if (!GROUP) {
+      own_part(v, own, acc[j]);
+#pragma unroll
+      for (int i = 0; i < VBITS; ++i) axpy(acc[j], a.cinside[i], flip_inside<CPLX>(own, i));
+    }
+#pragma unroll
+    for (int k = 0; k < kRegBits; ++k)
+      if (!GROUP || LOW + k >= a.lo) axpy(acc[j ^ (1 << k)], a.cbit[LOW + k], own);
+#pragma unroll
+    for (int i = 0; i < LOW; ++i)
+      if (!GROUP || i >= a.lo) axpy(acc[j], a.cbit[i], load_word(box + (v ^ (1 << i))));
+  }
+  return true;
+}
+
+// A block per contiguous box of 2^VB words (8 or 10), the flips of the `extra`
+// bits above the box from their partners' words in global memory. They come
+// after the box (which keeps the load pipe busier) or, with FAR_FIRST, before
+// it: FP32 sums then stay small until the diagonal, usually the largest term,
+// joins them, and their rounding error is a quarter smaller.
+template <typename T, bool CPLX, int VB, bool FAR_FIRST>
+__global__ void __launch_bounds__((1 << VB) / kWordsPerThread) flip_box_kernel(const __grid_constant__ BoxArgs<T> a) {
+  using W = Word<T>;
+  constexpr int VBITS = WordShape<T, CPLX>::VBITS;
+  constexpr int LOW = VB - kRegBits;
+  __shared__ __align__(128) W box[1 << VB];
+  __shared__ __align__(8) uint64_t full;
+  __shared__ double dword[1 << (VB - kBoxLaneBits)];
+  const uint64_t id = blockIdx.x;
+  if (threadIdx.x == 0) {
+    mbar_init(&full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(&full, 16u << VB);
+    bulk_load(box, a.x + (id << VB), 16u << VB, &full);
+  }
+  for (int u = threadIdx.x; u < (1 << (VB - kBoxLaneBits)); u += blockDim.x)
+    dword[u] = word_diagonal<T, VB, VBITS>(a, id, u);
   __syncthreads();
-  const uint64_t boxes = 1ull << (L - TB);
-  const uint64_t mine = boxes > blockIdx.x ? (boxes - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const E* x = static_cast<const E*>(a.x);
-  // global index of box position 0 and the box's load coordinates
-  const int batch_shift = GROUP ? a.b0 - R - a.bb : 0;  // bits of the batch coordinate above the box's batch
-  auto box_id = [&](uint64_t k) { return blockIdx.x + k * gridDim.x; };
-  auto issue = [&](uint64_t k) {
-    const uint64_t id = box_id(k);
-    E* dst = stage_buf + static_cast<size_t>(k % kStages) * kBox;
-    mbar_expect_tx(&full[k % kStages], kBox * static_cast<uint32_t>(sizeof(E)));
-    if (GROUP) {
-      // id = batch block (low b0 - R - bb bits) | above-group index
-      const uint64_t blk = id & ((1ull << batch_shift) - 1);
-      const uint64_t above = id >> batch_shift;
-      tensor_load5(dst, &map, static_cast<int>(blk << a.bb), static_cast<int>(above), &full[k % kStages]);
-    } else {
-      bulk_load(dst, x + (id << TB), kBox * static_cast<uint32_t>(sizeof(E)), &full[k % kStages]);
+  const uint64_t gbase = id << VB;
+  const uint64_t g0 = gbase | threadIdx.x;
+  W acc[kWordsPerThread];
+#pragma unroll
+  for (int j = 0; j < kWordsPerThread; ++j) {
+    if (a.q) acc[j] = kappa_word<CPLX>(a.kr, a.ki, load_word(a.q + g0 + (j << LOW)));
+    else acc[j].a = acc[j].b = 0;
+  }
+  if (a.p) {
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; ++j) axpy(acc[j], coef_of(a.gamma), load_word(a.p + g0 + (j << LOW)));
+  }
+  auto far_flips = [&] {
+#pragma unroll 1
+    for (int i = 0; i < a.extra; ++i) {
+      const W* partner = a.x + (g0 ^ (1ull << (VB + i)));
+#pragma unroll
+      for (int j = 0; j < kWordsPerThread; ++j) axpy(acc[j], a.cextra[i], load_word(partner + (j << LOW)));
     }
   };
-  if (threadIdx.x == 0)
-    for (uint64_t k = 0; k < mine && k < static_cast<uint64_t>(kStages); ++k) issue(k);
-  const T alpha = static_cast<T>(a.alpha), beta = static_cast<T>(a.beta), gamma = static_cast<T>(a.gamma);
-  const T kr = static_cast<T>(a.kr), ki = static_cast<T>(a.ki);
-  E* out = static_cast<E*>(a.out);
-  const E* pv = static_cast<const E*>(a.p);
-  const E* qv = static_cast<const E*>(a.q);
-  const T* low_table = static_cast<const T*>(a.low_table);
-  const int pos_shift = R + a.bb;  // group pass: box position bit of group bit 0
-  // flip coefficients of this pass in registers (TB low bits, or the group's bits)
-  constexpr int kFlips = GROUP ? TB - R : TB;
-  T coef[kFlips];
-#pragma unroll
-  for (int i = 0; i < kFlips; ++i) coef[i] = GROUP ? (i < a.G ? cx[a.b0 + i] : static_cast<T>(0)) : cx[i];
-  for (uint64_t k = 0; k < mine; ++k) {
-    const uint64_t id = box_id(k);
-    E* box = stage_buf + static_cast<size_t>(k % kStages) * kBox;
-    // Global index of each of this thread's elements, and the operands that
-    // come from global memory, loaded before the wait on the box so that
-    // their latency overlaps the copy.
-    uint64_t sidx[kPer];
-    E pre0[kPer], pre1[kPer];
-    T lowv[kPer];
-    if (GROUP) {
-      const uint64_t blk = id & ((1ull << batch_shift) - 1);
-      const uint64_t above = id >> batch_shift;
-      const uint64_t base = (blk << (a.bb + R)) | (above << (a.b0 + a.G));
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int e = threadIdx.x + u * kPassThreads;
-        sidx[u] = base | static_cast<uint64_t>(e & ((1 << pos_shift) - 1)) |
-                  (static_cast<uint64_t>(e >> pos_shift) << a.b0);
-        pre0[u] = out[sidx[u]];
-      }
-    } else {
-      const uint64_t base = id << TB;
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int j = threadIdx.x + u * kPassThreads;
-        sidx[u] = base + j;
-        lowv[u] = __ldg(low_table + j);
-        pre0[u] = pv ? pv[sidx[u]] : zero_elem<E>();
-        pre1[u] = qv ? qv[sidx[u]] : zero_elem<E>();
-      }
-      if (threadIdx.x == 0) d_high = static_cast<const T*>(a.high_table)[id];
-    }
-    if (threadIdx.x == 0 && !mbar_wait(&full[k % kStages], static_cast<uint32_t>((k / kStages) & 1))) {
-      atomicExch(a.status, 1);
-      abort_flag = 1;
-      failed_box = k;
-    }
-    __syncthreads();
-    if (abort_flag) break;
-    if (GROUP) {
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int e = threadIdx.x + u * kPassThreads;
-        E acc = zero_elem<E>();
-#pragma unroll
-        for (int i = 0; i < kFlips; ++i)
-          if (i < a.G) acc = scale_add(acc, coef[i], box[e ^ (1 << (pos_shift + i))]);
-        out[sidx[u]] = add(pre0[u], scaled(alpha, acc));
-      }
-    } else {
-      const T dh = d_high;
-      const int nc = n_cross;
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int j = threadIdx.x + u * kPassThreads;
-        const uint64_t s = sidx[u];
-        T d = dh + lowv[u];
-        for (int c = 0; c < nc; ++c) d += (__popcll(~s & cross_mask[c]) & 1) ? -cross_coef[c] : cross_coef[c];
-        const E xs = box[j];
-        E acc = scaled(d, xs);
-#pragma unroll
-        for (int i = 0; i < kFlips; ++i) acc = scale_add(acc, coef[i], box[j ^ (1 << i)]);
-        E o = add(scaled(alpha, acc), scaled(beta, xs));
-        if (pv) o = add(o, scaled(gamma, pre0[u]));
-        if (qv) o = add(o, kappa_times(kr, ki, pre1[u]));
-        out[s] = o;
-      }
-    }
-    __syncthreads();  // every thread is done with this stage (and with d_high)
-    if (threadIdx.x == 0 && k + kStages < mine) issue(k + kStages);
+  if (FAR_FIRST) far_flips();
+  const BoxDiagonal<T, CPLX, VB> diagonal(a);
+  if (!box_flips<T, CPLX, VB, false>(
+          a, box, static_cast<int>(threadIdx.x), [&](int j) { return j > 0 || mbar_wait(&full, 0); },
+          [&](int v, const W& own, W& sum) { diagonal.add(a, gbase, dword, v, own, sum); }, acc)) {
+    // the copy may still be in flight: one more bounded wait before the box is given up
+    atomicExch(a.status, 1);
+    mbar_wait(&full, 0);
+    return;
   }
-  // after a time-out, wait (bounded) for the copies still in flight (the box
-  // that timed out and the one issued after it) before leaving
-  if (threadIdx.x == 0 && abort_flag)
-    for (uint64_t k = failed_box; k < mine && k < failed_box + kStages; ++k)
-      mbar_wait(&full[k % kStages], static_cast<uint32_t>((k / kStages) & 1));
+  if (!FAR_FIRST) far_flips();
+#pragma unroll
+  for (int j = 0; j < kWordsPerThread; ++j) {
+    store_word(a.out + g0 + (j << LOW), acc[j]);
+  }
+}
+
+// A group pass: a block per box of 64 KB (12 word bits), three resident per SM,
+// in two trips of eight words per thread. The box arrives in eighths (the top
+// three word bits), each on its own barrier, so that a block's arithmetic
+// overlaps its own copy: blocks that started together would otherwise load,
+// compute and store in step. out is requested before the first wait.
+constexpr int kPassTrips = 2;
+constexpr int kPassThreads = (1 << kBoxMaxWords) / (kWordsPerThread * kPassTrips);
+
+template <typename T, bool CPLX>
+__global__ void __launch_bounds__(kPassThreads, 3) flip_group_kernel(const __grid_constant__ CUtensorMap map,
+                                                                     const __grid_constant__ BoxArgs<T> a) {
+  using W = Word<T>;
+  constexpr int VB = kBoxMaxWords;
+  constexpr int VBITS = WordShape<T, CPLX>::VBITS;
+  constexpr int LOW = VB - kRegBits;
+  constexpr uint32_t kPart = 16u << LOW;  // bytes of an eighth
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  W* box = reinterpret_cast<W*>(smem_raw);
+  __shared__ __align__(8) uint64_t full[kWordsPerThread];
+  // box id = batch block (low bits) | index above the group
+  const int run_bits = 2 + a.bb;
+  const int batch_shift = a.b0 - VBITS - run_bits;
+  const uint64_t blk = blockIdx.x & ((1ull << batch_shift) - 1), above = static_cast<uint64_t>(blockIdx.x) >> batch_shift;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; ++j) mbar_init(&full[j], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; ++j) {
+      mbar_expect_tx(&full[j], kPart);
+      tensor_load5(box + (j << LOW), &map, static_cast<int>(blk << a.bb), j, static_cast<int>(above), &full[j]);
+    }
+  }
+  __syncthreads();
+  const uint64_t gbase = (blk << run_bits) | (above << (a.b0 + a.G - VBITS));
+  // global word of box word v
+  auto global_word = [&](int v) -> uint64_t {
+    return gbase | static_cast<uint64_t>(v & ((1 << run_bits) - 1)) |
+           (static_cast<uint64_t>(v >> run_bits) << (a.b0 - VBITS));
+  };
+#pragma unroll 1
+  for (int trip = 0; trip < kPassTrips; ++trip) {
+    const int v0 = static_cast<int>(threadIdx.x) | (trip * kPassThreads);
+    W acc[kWordsPerThread], before[kWordsPerThread];
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; ++j) {
+      before[j] = load_early(a.out + global_word(v0 | (j << LOW)));
+      acc[j].a = acc[j].b = 0;
+    }
+    if (!box_flips<T, CPLX, VB, true>(
+            a, box, v0, [&](int j) { return trip > 0 || mbar_wait(&full[j], 0); }, [](int, const W&, W&) {}, acc)) {
+      // copies may still be in flight: one more bounded wait for each before the box is given up
+      atomicExch(a.status, 1);
+      for (int j = 0; j < kWordsPerThread; ++j) mbar_wait(&full[j], 0);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; ++j) {
+      axpy(acc[j], coef_of(static_cast<T>(1)), before[j]);
+      store_word(a.out + global_word(v0 | (j << LOW)), acc[j]);
+    }
+  }
 }
 
 // Self-test of the bounded stage wait: one thread arms an mbarrier for bytes
@@ -453,15 +658,16 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // Tensor map of the group boxes over x (4-byte units): d0 the 64-byte run
-// (R bits), d1 the bits between the run and the group (box: bb of them),
-// d2 / d3 the group's bits (at most 8 per dimension), d4 the bits above.
+// (R bits), d1 the bits between the run and the group (box: bb of them), d2
+// the group's bits below its top three (at most 7), d3 the top three (one
+// eighth of a box per copy), d4 the bits above.
 CUtensorMap group_map(const void* x, int sites, int esize, int r, int b0, int G, int bb) {
-  const int g1 = std::min(G, 8), g2 = G - g1;
-  const cuuint64_t dims[5] = {static_cast<cuuint64_t>((esize << r) / 4), 1ull << (b0 - r), 1ull << g1, 1ull << g2,
+  const int g1 = G - 3;
+  const cuuint64_t dims[5] = {static_cast<cuuint64_t>((esize << r) / 4), 1ull << (b0 - r), 1ull << g1, 8ull,
                               1ull << (sites - b0 - G)};
   const cuuint64_t strides[4] = {static_cast<cuuint64_t>(esize) << r, static_cast<cuuint64_t>(esize) << b0,
                                  static_cast<cuuint64_t>(esize) << (b0 + g1), static_cast<cuuint64_t>(esize) << (b0 + G)};
-  const cuuint32_t box[5] = {static_cast<cuuint32_t>((esize << r) / 4), 1u << bb, 1u << g1, 1u << g2, 1u};
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>((esize << r) / 4), 1u << bb, 1u << g1, 1u, 1u};
   const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
   CUtensorMap map;
   const CUresult rc = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 5, const_cast<void*>(x), dims, strides,
@@ -471,14 +677,42 @@ CUtensorMap group_map(const void* x, int sites, int esize, int r, int b0, int G,
   return map;
 }
 
-// Chooses between the one-pass kernel and the multi-pass action: QMBED_FLIP_PASSES=single|multi
-// forces one (tests); otherwise vectors beyond 256 MB take the multi-pass action.
-bool use_multipass(uint64_t n, int esize, int sites, int tb) {
-  if (const char* env = std::getenv("QMBED_FLIP_PASSES")) {
-    if (std::strcmp(env, "single") == 0) return false;
-    if (std::strcmp(env, "multi") == 0) return sites > tb;
-  }
-  return sites > tb && n * static_cast<uint64_t>(esize) >= (256ull << 20);
+// One launch while the partners above the box come from the L2. Vectors from
+// 512 MB on (256 MB when p or q stream beside them) take their top nine bits
+// in a group pass instead: complex64 H.v of 25 sites (268 MB) 292 us in one
+// launch against 307 with a group pass and 631 against 630 at 26 sites; with p
+// and q 351 against 329 at 25 sites and 167 against 172 at 24.
+constexpr uint64_t kGroupPassBytes = 512ull << 20, kGroupPassBytesPq = 256ull << 20;
+// Bits of a group pass (of 7 to 10, 9 is fastest or within 3% of it from 24 to
+// 28 sites: longer runs against fewer direct reads) and the most bits read
+// directly beside one (a window of 2^10 boxes, 16 MB) before another pass.
+constexpr int kGroupBits = 9, kDirectBits = 10;
+
+// QMBED_FLIP_PASSES=single|multi forces flip_chain_kernel or group passes (tests).
+BoxPlan box_plan(int sites, int vbits, uint64_t bytes, bool pq) {
+  BoxPlan plan;
+  const char* env = std::getenv("QMBED_FLIP_PASSES");
+  const bool single = env && std::strcmp(env, "single") == 0, multi = env && std::strcmp(env, "multi") == 0;
+  const int words = sites - vbits;  // word bits of the whole vector
+  if (single || words < 8 || (multi && words <= kBoxMaxWords)) return plan;
+  // 4 KB boxes while 16 KB boxes would leave SMs without work
+  plan.vb = words >= 17 ? 10 : 8;
+  plan.extra = words - plan.vb;
+  if (multi) plan.vb = 10;
+  // Separate passes used to sum the flips of FP32 vectors from 256 MB on:
+  // complex64 of 25 sites has 0.94e-7 of relative error in that form, 0.89e-7
+  // with the far flips first (286 us) and 1.19e-7 with them last (258 us).
+  // Below, the order of the one-pass kernel had 1.19e-7 at 24 sites, now 1.16e-7.
+  plan.far_first = bytes >= (256ull << 20);
+  const bool passes = multi || bytes >= (pq ? kGroupPassBytesPq : kGroupPassBytes);
+  if (!passes) return plan;
+  plan.extra = words - plan.vb;
+  do {
+    const int g = std::min(plan.extra, kGroupBits);
+    plan.groups.push_back(g);
+    plan.extra -= g;
+  } while (plan.extra > kDirectBits);
+  return plan;
 }
 
 }  // namespace
@@ -498,6 +732,7 @@ FlipChain::FlipChain(const FlipChainDesc& d) : sites_(d.sites), n_diag_(static_c
     QMBED_CUDA(cudaMemcpy(diag_coefs_.get(), d.z_coefs.data(), n_diag_ * sizeof(double), cudaMemcpyHostToDevice));
   }
   QMBED_CUDA(cudaMemcpy(x_coefs_.get(), x.data(), 64 * sizeof(double), cudaMemcpyHostToDevice));
+  host_diag_masks_ = d.z_masks;
   host_diag_coefs_ = d.z_coefs;
   host_x_ = x;
 }
@@ -512,6 +747,20 @@ double FlipChain::norm_bound() const {
 void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
                       const FlipStep& step, cudaStream_t stream) const {
   const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1);
+  {
+    const int vbits = log2_int(16 / esize);
+    const BoxPlan plan = box_plan(sites_, vbits, dim() * static_cast<uint64_t>(esize), p || q);
+    auto aligned = [](const void* ptr) { return ptr == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
+    if (plan.vb > 0 && aligned(x) && aligned(out) && aligned(p) && aligned(q)) {
+      const bool over = x == out || (q && q == out);
+      if (over && dim() * static_cast<uint64_t>(esize) >= (256ull << 20))
+        raise(QMBED_INVALID_OPTIONS, "the flip-chain action cannot write over x or q");
+      if (!over) {
+        apply_boxes(precision, cplx, x, out, p, q, step, stream, plan);
+        return;
+      }
+    }
+  }
   const int tbits = log2_int(kTileBytes / esize);
   const int tb = std::min(sites_, tbits);
   const uint64_t n = dim();
@@ -539,15 +788,6 @@ void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const 
     QMBED_LAUNCH_CHECK();
     tables_ready_ |= table_slot;
     table_tb_[table_slot - 1] = tb;
-  }
-  // TMA boxes (cp.async.bulk needs 16-byte aligned sources; tensor maps
-  // 16-byte aligned bases): vectors that start elsewhere, such as offset
-  // views, take the one-pass kernel
-  auto aligned = [](const void* ptr) { return ptr == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 31) == 0; };
-  if (aligned(x) && aligned(out) && aligned(p) && aligned(q) &&
-      use_multipass(n, esize, sites_, log2_int(kBoxBytes / esize))) {
-    apply_multipass(precision, cplx, x, out, p, q, step, stream, sms);
-    return;
   }
   const size_t smem = static_cast<size_t>(esize) << tb;
   const int grid = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(n >> tb, 3ull * sms)));
@@ -577,29 +817,47 @@ namespace qmbed {
 
 namespace {
 
-template <typename T, bool C, int TB, int R>
-void run_passes(int sites, const PassArgs& base, int esize, cudaStream_t stream, int sms) {
-  const size_t smem = static_cast<size_t>(kStages) * kBoxBytes;
-  auto pass_a = flip_pass_kernel<T, C, TB, R, false>;
-  auto pass_g = flip_pass_kernel<T, C, TB, R, true>;
-  QMBED_CUDA(cudaFuncSetAttribute(pass_a, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  QMBED_CUDA(cudaFuncSetAttribute(pass_g, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  int per_sm = 1;
-  QMBED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_a, kPassThreads, smem));
-  const uint64_t boxes = 1ull << (sites - TB);
-  const unsigned grid =
-      static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(boxes, static_cast<uint64_t>(sms) * std::max(per_sm, 1))));
-  CUtensorMap unused{};
-  pass_a<<<grid, kPassThreads, smem, stream>>>(unused, base);
+template <typename T>
+typename Coef<T>::type host_coef(double c) {
+  const T v = static_cast<T>(c);
+  typename Coef<T>::type r;
+  for (size_t i = 0; i < sizeof(r) / sizeof(T); ++i)
+    std::memcpy(reinterpret_cast<unsigned char*>(&r) + i * sizeof(T), &v, sizeof(T));
+  return r;
+}
+
+template <typename T, bool C>
+void launch_box_plan(BoxArgs<T> base, const BoxPlan& plan, double alpha, const std::vector<double>& xc, int sites,
+                     cudaStream_t stream) {
+  constexpr int VBITS = WordShape<T, C>::VBITS;
+  base.sites = sites;
+  base.extra = plan.extra;
+  for (int i = 0; i < plan.vb; ++i) base.cbit[i] = host_coef<T>(alpha * xc[VBITS + i]);
+  for (int i = 0; i < VBITS; ++i) base.cinside[i] = host_coef<T>(alpha * xc[i]);
+  for (int i = 0; i < plan.extra; ++i) base.cextra[i] = host_coef<T>(alpha * xc[VBITS + plan.vb + i]);
+  const unsigned boxes = 1u << (sites - VBITS - plan.vb);
+  if (plan.vb == 8) flip_box_kernel<T, C, 8, false><<<boxes, 32, 0, stream>>>(base);
+  else if (plan.far_first) flip_box_kernel<T, C, 10, sizeof(T) == 4><<<boxes, 128, 0, stream>>>(base);
+  else flip_box_kernel<T, C, 10, false><<<boxes, 128, 0, stream>>>(base);
   QMBED_LAUNCH_CHECK();
-  for (int b0 = TB; b0 < sites;) {
-    const int G = std::min(TB - R, sites - b0);
-    PassArgs g = base;
-    g.b0 = b0;
-    g.G = G;
-    g.bb = TB - R - G;
-    const CUtensorMap map = group_map(base.x, sites, esize, R, b0, G, g.bb);
-    pass_g<<<grid, kPassThreads, smem, stream>>>(map, g);
+  if (plan.groups.empty()) return;
+  constexpr int kSmem = 16 << kBoxMaxWords;
+  auto group = flip_group_kernel<T, C>;
+  QMBED_CUDA(cudaFuncSetAttribute(group, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  int b0 = VBITS + plan.vb + plan.extra;
+  for (int G : plan.groups) {
+    BoxArgs<T> g = base;
+    // a box's eighths are its group's top three bits: a smaller group takes
+    // the bits below it along, without their flips
+    const int skip = std::max(0, 3 - G);
+    g.b0 = b0 - skip;
+    g.G = G + skip;
+    g.bb = kBoxMaxWords - 2 - g.G;
+    g.lo = kBoxMaxWords - G;
+    for (int i = g.lo; i < kBoxMaxWords; ++i) g.cbit[i] = host_coef<T>(alpha * xc[b0 + i - g.lo]);
+    const CUtensorMap map =
+        group_map(base.x, sites, static_cast<int>(sizeof(T)) * (C ? 2 : 1), VBITS + 2, g.b0, g.G, g.bb);
+    group<<<1u << (sites - VBITS - kBoxMaxWords), kPassThreads, kSmem, stream>>>(map, g);
     QMBED_LAUNCH_CHECK();
     b0 += G;
   }
@@ -607,62 +865,90 @@ void run_passes(int sites, const PassArgs& base, int esize, cudaStream_t stream,
 
 }  // namespace
 
-void FlipChain::apply_multipass(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
-                                const FlipStep& step, cudaStream_t stream, int sms) const {
-  if (x == out || (q && q == out)) raise(QMBED_INVALID_OPTIONS, "the flip-chain action cannot write over x or q");
-  const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1);
-  const int tb = log2_int(kBoxBytes / esize);
-  // the low-bit diagonal table of this box width
-  const size_t need = static_cast<size_t>(esize / (cplx ? 2 : 1)) << tb;
-  const int slot = precision == 64 ? 0 : 1;
-  const size_t high_need = static_cast<size_t>(esize / (cplx ? 2 : 1)) << (sites_ - tb);
-  if (pass_table_bytes_[slot] < need || pass_table_tb_[slot] != tb) {
-    pass_tables_[slot].allocate(need);
-    pass_high_tables_[slot].allocate(high_need);
-    pass_table_bytes_[slot] = need;
-    pass_table_tb_[slot] = tb;
-    const int blocks = static_cast<int>(std::min<uint64_t>(((1ull << tb) + 255) / 256, 1024));
-    const int hblocks = static_cast<int>(std::min<uint64_t>(((1ull << (sites_ - tb)) + 255) / 256, 4096));
-    if (precision == 64) {
-      diag_low_table_kernel<double><<<blocks, 256, 0, stream>>>(tb, n_diag_, diag_masks_.as<uint64_t>(),
-                                                                diag_coefs_.as<double>(), pass_tables_[slot].as<double>());
-      diag_high_table_kernel<double><<<hblocks, 256, 0, stream>>>(tb, sites_, n_diag_, diag_masks_.as<uint64_t>(),
-                                                                  diag_coefs_.as<double>(),
-                                                                  pass_high_tables_[slot].as<double>());
-    } else {
-      diag_low_table_kernel<float><<<blocks, 256, 0, stream>>>(tb, n_diag_, diag_masks_.as<uint64_t>(),
-                                                               diag_coefs_.as<double>(), pass_tables_[slot].as<float>());
-      diag_high_table_kernel<float><<<hblocks, 256, 0, stream>>>(tb, sites_, n_diag_, diag_masks_.as<uint64_t>(),
-                                                                 diag_coefs_.as<double>(),
-                                                                 pass_high_tables_[slot].as<float>());
+// The diagonal's tables for boxes of 2^vb words, built once per (precision,
+// real or complex); complete before any stream can use them.
+const FlipChain::BoxTables& FlipChain::box_tables(int precision, bool cplx, int vb, cudaStream_t stream) const {
+  const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1), vbits = log2_int(16 / esize);
+  std::lock_guard<std::mutex> lock(tables_mu_);
+  BoxTables& t = box_tables_[(precision == 64 ? 0 : 2) + (cplx ? 1 : 0)][vb == 10 ? 1 : 0];
+  if (t.ready) return t;
+  const uint64_t lanes = (1ull << (kBoxLaneBits + vbits)) - 1, in_box = (1ull << (vb + vbits)) - 1;
+  const uint64_t words = in_box & ~lanes;
+  const int n_lanes = 1 << (kBoxLaneBits + vbits), n_words = 1 << (vb - kBoxLaneBits);
+  std::vector<double> table(static_cast<size_t>(n_lanes + n_words), 0.0);
+  std::vector<uint64_t> masks[2];
+  std::vector<double> coefs[2];
+  for (size_t k = 0; k < host_diag_masks_.size(); ++k) {
+    const uint64_t m = host_diag_masks_[k];
+    const double c = host_diag_coefs_[k];
+    auto sign = [&](uint64_t s) { return (__builtin_popcountll(~s & m) & 1) ? -c : c; };
+    if ((m & ~lanes) == 0) {
+      for (int i = 0; i < n_lanes; ++i) table[i] += sign(static_cast<uint64_t>(i));
+    } else if ((m & ~words) == 0) {
+      for (int u = 0; u < n_words; ++u) table[n_lanes + u] += sign(static_cast<uint64_t>(u) << (kBoxLaneBits + vbits));
+    } else if ((m & in_box) != 0) {
+      const int list = (m & lanes) != 0 ? 0 : 1;
+      masks[list].push_back(m);
+      coefs[list].push_back(c);
     }
-    QMBED_LAUNCH_CHECK();
   }
-  PassArgs a{};
-  a.sites = sites_;
-  a.nd = n_diag_;
-  a.masks = diag_masks_.as<uint64_t>();
-  a.coefs = diag_coefs_.as<double>();
-  a.low_table = pass_tables_[slot].get();
-  a.high_table = pass_high_tables_[slot].get();
-  a.xcoef = x_coefs_.as<double>();
-  a.x = x;
-  a.out = out;
-  a.p = p;
-  a.q = q;
-  a.alpha = step.alpha;
-  a.beta = step.beta;
-  a.gamma = step.gamma;
-  a.kr = step.kappa_re;
-  a.ki = step.kappa_im;
-  a.status = status_.as<int>();
-  if (precision == 64) {
-    if (cplx) run_passes<double, true, 11, 2>(sites_, a, esize, stream, sms);
-    else run_passes<double, false, 12, 3>(sites_, a, esize, stream, sms);
-  } else {
-    if (cplx) run_passes<float, true, 12, 3>(sites_, a, esize, stream, sms);
-    else run_passes<float, false, 13, 4>(sites_, a, esize, stream, sms);
+  t.n_lane = static_cast<int>(masks[0].size());
+  t.n_word = static_cast<int>(masks[1].size());
+  masks[0].insert(masks[0].end(), masks[1].begin(), masks[1].end());
+  coefs[0].insert(coefs[0].end(), coefs[1].begin(), coefs[1].end());
+  const uint64_t boxes = 1ull << (sites_ - vbits - vb);
+  // [span masks][span coefs][lane table, word table][high table], FP64
+  const size_t spans = std::max<size_t>(masks[0].size(), 1) * 8;
+  t.at_coefs = spans;
+  t.at_table = 2 * spans;
+  t.at_words = t.at_table + static_cast<size_t>(n_lanes) * 8;
+  t.at_high = t.at_words + static_cast<size_t>(n_words) * 8;
+  std::vector<unsigned char> image(t.at_high, 0);
+  if (!masks[0].empty()) {
+    std::memcpy(image.data(), masks[0].data(), masks[0].size() * 8);
+    std::memcpy(image.data() + t.at_coefs, coefs[0].data(), coefs[0].size() * 8);
   }
+  std::memcpy(image.data() + t.at_table, table.data(), table.size() * 8);
+  t.buf.allocate(t.at_high + boxes * 8);
+  QMBED_CUDA(cudaMemcpyAsync(t.buf.get(), image.data(), image.size(), cudaMemcpyHostToDevice, stream));
+  const int blocks = static_cast<int>(std::min<uint64_t>((boxes + 255) / 256, 4096));
+  diag_high_table_kernel<<<blocks, 256, 0, stream>>>(vb + vbits, sites_, n_diag_, diag_masks_.as<uint64_t>(),
+                                                     diag_coefs_.as<double>(),
+                                                     reinterpret_cast<double*>(t.buf.as<unsigned char>() + t.at_high));
+  QMBED_LAUNCH_CHECK();
+  QMBED_CUDA(cudaStreamSynchronize(stream));
+  t.ready = true;
+  return t;
+}
+
+void FlipChain::apply_boxes(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
+                            const FlipStep& step, cudaStream_t stream, const BoxPlan& plan) const {
+  const BoxTables& t = box_tables(precision, cplx, plan.vb, stream);
+  unsigned char* base = t.buf.as<unsigned char>();
+  auto run = [&](auto ttag, auto ctag) {
+    using T = decltype(ttag);
+    BoxArgs<T> a{};
+    a.lane_table = reinterpret_cast<const double*>(base + t.at_table);
+    a.word_table = reinterpret_cast<const double*>(base + t.at_words);
+    a.high_table = reinterpret_cast<const double*>(base + t.at_high);
+    a.span_masks = reinterpret_cast<const uint64_t*>(base);
+    a.span_coefs = reinterpret_cast<const double*>(base + t.at_coefs);
+    a.n_lane = t.n_lane;
+    a.n_word = t.n_word;
+    a.x = static_cast<const Word<T>*>(x);
+    a.out = static_cast<Word<T>*>(out);
+    a.p = static_cast<const Word<T>*>(p);
+    a.q = static_cast<const Word<T>*>(q);
+    a.alpha = step.alpha;
+    a.beta = step.beta;
+    a.gamma = static_cast<T>(step.gamma);
+    a.kr = static_cast<T>(step.kappa_re);
+    a.ki = static_cast<T>(step.kappa_im);
+    a.status = status_.as<int>();
+    launch_box_plan<T, decltype(ctag)::value>(a, plan, step.alpha, host_x_, sites_, stream);
+  };
+  if (precision == 64) cplx ? run(double{}, std::true_type{}) : run(double{}, std::false_type{});
+  else cplx ? run(float{}, std::true_type{}) : run(float{}, std::false_type{});
 }
 
 void FlipChain::check_status() const {

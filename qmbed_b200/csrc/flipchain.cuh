@@ -1,13 +1,13 @@
 // Structured action of full-space spin-1/2 chains whose terms are products of
 // z (diagonal) or a single x (one bit flip): transverse-field Ising chains and
 // their relatives. No matrix is stored: the diagonal is evaluated from the bits
-// of the state index, and one pass over shared-memory tiles of consecutive
-// elements serves the low-bit flips from the tile and the high-bit flips from
-// coalesced reads of the partner tiles.
+// of the state index and the flips are served from boxes of the vector in shared
+// memory, in one pass or in one pass per group of bits.
 #pragma once
 
 #include <complex>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -34,6 +34,16 @@ struct FlipStep {
 // completes (1024 polls) on `device`; returns 1 when it gave up as designed.
 int flip_stage_wait_selftest(int device);
 
+// How an application runs: word bits of its boxes (0: one tile per block),
+// flips above the box that read their partners directly, and the bits of the
+// group passes, lowest first.
+struct BoxPlan {
+  int vb = 0;
+  int extra = 0;
+  std::vector<int> groups;
+  bool far_first = false;  // FP32: the direct flips before the box's
+};
+
 class FlipChain {
  public:
   explicit FlipChain(const FlipChainDesc& d);
@@ -55,13 +65,20 @@ class FlipChain {
   mutable size_t tables_bytes_ = 0;
   mutable int tables_ready_ = 0;  // bit 1: FP64 table, bit 2: FP32 table
   mutable int table_tb_[2] = {0, 0};
-  // multi-pass action (vectors beyond the L2): low-bit tables of its box width, time-out status
-  void apply_multipass(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
-                       const FlipStep& step, cudaStream_t stream, int sms) const;
-  mutable DeviceBuffer pass_tables_[2], pass_high_tables_[2];
-  mutable size_t pass_table_bytes_[2] = {0, 0};
-  mutable int pass_table_tb_[2] = {0, 0};
+  // Box action and the diagonal's tables per box width.
+  struct BoxTables {
+    bool ready = false;
+    DeviceBuffer buf;
+    size_t at_coefs = 0, at_table = 0, at_words = 0, at_high = 0;
+    int n_lane = 0, n_word = 0;
+  };
+  const BoxTables& box_tables(int precision, bool cplx, int vb, cudaStream_t stream) const;
+  void apply_boxes(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
+                   const FlipStep& step, cudaStream_t stream, const BoxPlan& plan) const;
+  mutable std::mutex tables_mu_;
+  mutable BoxTables box_tables_[4][2];  // [precision, complex][box width]
   DeviceBuffer status_;
+  std::vector<uint64_t> host_diag_masks_;
   std::vector<double> host_diag_coefs_, host_x_;
 };
 

@@ -1090,7 +1090,7 @@ void SpinOperator::build_instances(const std::vector<TermDesc>& terms, const Ope
   if (basis_->words() == 1) {
     host_prog_ = std::make_unique<FlipProgram>(compile_flip_program(adj, factors_, sites, basis_->params().up >= 0));
     prog_.upload(*host_prog_);
-    hermitian_terms_ = checks.hermiticity && hermitian_by_terms(adj, fwd, factors_, sites);
+    hermitian_terms_ = checks.hermiticity && !flip_ && hermitian_by_terms(adj, fwd, factors_, sites);
   }
   inst_adj_.allocate(std::max<size_t>(adj.size(), 1) * sizeof(Instance));
   inst_fwd_.allocate(std::max<size_t>(fwd.size(), 1) * sizeof(Instance));
