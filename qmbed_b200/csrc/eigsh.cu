@@ -28,6 +28,9 @@ constexpr size_t kGuaranteedDense = 128;
 constexpr size_t kAutomaticDense = 256;
 constexpr size_t kFullKrylovDenseFallback = 2048;
 constexpr size_t kTridiagonalWindow = 96;
+// Lanczos steps queued before the host reads their records: a run that ends
+// early has at most this many steps to throw away.
+constexpr size_t kQueuedSteps = 32;
 constexpr double kEps = 2.220446049250313e-16;
 const double kDgks = 1.0 / std::sqrt(2.0);
 // FP32 vectors resolve residuals to about 1e-7 of the spectral scale; the mixed
@@ -114,6 +117,12 @@ struct Ortho {
   std::vector<C64> projection;
 };
 
+Ortho from_record(const OrthoRecord& r, int projection_from) {
+  Ortho out{r.ok, static_cast<size_t>(r.second ? 2 : 1), static_cast<size_t>(r.second ? 1 : 0), {}};
+  out.projection.assign(r.h.begin() + projection_from, r.h.end());
+  return out;
+}
+
 // orthonormalize_*_with_projection (src/solve/mod.rs:1520-1642): remove the
 // first `ncols` panel columns (locked then basis) from w, a DGKS second pass
 // when the norm drops below 1/sqrt(2), then normalise.
@@ -125,6 +134,15 @@ Ortho orthonormalize(Ctx& c, const Panel& Q, int ncols, int projection_from, con
   std::vector<C64> h(std::max(ncols, 1));
   double before, norm;
   const bool fused = c.prec == 64 && Q.n == c.n;
+  if (ncols > 0 && fused && c.ops.fused().applies(c.n, ncols)) {
+    // one launch: both passes, the norm and the scaled result
+    std::vector<OrthoRecord> records;
+    c.ops.fused().begin(1, ncols, 0.0, c.ops.stream());
+    c.ops.fused().step(static_cast<const double*>(Q.col(0)), c.n, ncols, static_cast<const double*>(src),
+                       static_cast<double*>(w), static_cast<double*>(slot), c.cplx, false, c.ops.stream());
+    c.ops.fused().finish(records, c.ops.stream());
+    return from_record(records[0], projection_from);
+  }
   if (ncols > 0 && fused) {
     // overlaps, subtraction and both norms in two sweeps and one synchronisation
     double before_sq = 0.0, norm_sq = 0.0;
@@ -241,7 +259,37 @@ EigshResult lanczos_window(Ctx& c, const EigshOptions& o, const void* initial_de
   }
   std::vector<double> alphas, betas;
   size_t passes = 0, seconds = 0, size = 0;
-  for (size_t it = 0; it < krylov; ++it) {
+  // FP64 steps queue up to kQueuedSteps at a time; the loop below takes over
+  // where a step needs a second pass that the queue does not make, and for FP32.
+  size_t begin = 0;
+  bool finished = false;
+  while (c.prec == 64 && begin < krylov && !finished) {
+    const size_t end = std::min(krylov, begin + kQueuedSteps);
+    c.ops.lanczos_begin(static_cast<int>(end - begin), static_cast<int>(end), begin > 0 ? betas[begin - 1] : 0.0);
+    for (size_t it = begin; it < end; ++it) {
+      c.apply(V.col(static_cast<int>(it)), out);
+      c.ops.lanczos_step(static_cast<const double*>(V.col(0)), n, static_cast<int>(it + 1), static_cast<double*>(out),
+                         it + 1 < krylov ? static_cast<double*>(V.col(static_cast<int>(it + 1))) : nullptr, c.cplx);
+    }
+    std::vector<OrthoRecord> records;
+    c.ops.lanczos_finish(records);
+    const bool whole = c.ops.lanczos_fused(n, static_cast<int>(end));
+    size_t it = begin;
+    for (; it < end && !finished; ++it) {
+      const OrthoRecord& r = records[it - begin];
+      if (r.second && !whole) break;  // redone below from this step on
+      alphas.push_back(r.h.back().real());
+      size = it + 1;
+      passes += r.second ? 2 : 1;
+      seconds += r.second ? 1 : 0;
+      if (it + 1 == krylov || r.norm <= 1.0e-14) finished = true;
+      else betas.push_back(r.norm);
+    }
+    c.applications -= end - it;
+    begin = it;
+    if (it < end) break;
+  }
+  for (size_t it = begin; it < krylov && !finished; ++it) {
     c.apply(V.col(static_cast<int>(it)), out);
     const int m = static_cast<int>(it + 1);
     double alpha, before, beta;
@@ -429,6 +477,39 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
       }
     }
     int cursor = known;
+    // The cycle's steps are queued on the assumption that every direction is
+    // accepted; from the first that is not, the loop below goes on step by step.
+    if (c.prec == 64 && c.ops.fused().applies(n, l + m) && cursor < b && a < m) {
+      c.ops.fused().begin(m - a, l + m, 0.0, c.ops.stream());
+      size_t queued = 0;
+      for (int qb = b, qa = a, qc = cursor; qc < qb && iterations + queued < o.max_iterations && qa < m; ++qc) {
+        c.apply(Q.col(l + qc), W.col(qa));
+        ++queued;
+        ++qa;
+        c.ops.fused().step(static_cast<const double*>(Q.col(0)), n, l + qb, static_cast<const double*>(W.col(qa - 1)),
+                           static_cast<double*>(tmp), qb < m ? static_cast<double*>(Q.col(l + qb)) : nullptr, c.cplx,
+                           false, c.ops.stream());
+        if (qb < m) ++qb;
+      }
+      std::vector<OrthoRecord> records;
+      c.ops.fused().finish(records, c.ops.stream());
+      size_t used = 0;
+      bool accepted = true;
+      for (; used < queued && accepted; ++used) {
+        const Ortho r = from_record(records[used], l);
+        ++iterations;
+        ++a;
+        passes += r.passes;
+        seconds += r.second_passes;
+        projection_columns.emplace_back(r.projection.begin(), r.projection.begin() + cursor + 1);
+        if (b < m) {
+          accepted = r.ok;
+          if (r.ok) ++b;
+        }
+        ++cursor;
+      }
+      c.applications -= queued - used;
+    }
     while (cursor < b && iterations < o.max_iterations && a < m) {
       c.apply(Q.col(l + cursor), W.col(a));
       ++iterations;

@@ -863,7 +863,8 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 enum { kReal = 0, kRealPair = 1, kComplex = 2 };
 template <int MODE>
 __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const double* __restrict__ Q, uint64_t n, int m,
-                                                                      const double* __restrict__ h, double beta,
+                                                                      const double* __restrict__ h, double beta_value,
+                                                                      const double* __restrict__ beta_device,
                                                                       int before_mode, const double* src,
                                                                       double* w, double* __restrict__ partials) {
   extern __shared__ double hs[];
@@ -871,6 +872,7 @@ __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const d
   for (int t = threadIdx.x; t < 2 * m; t += blockDim.x) hs[t] = h[t];
   __syncthreads();
   const double alpha = hs[2 * (m - 1)];
+  const double beta = beta_device ? *beta_device : beta_value;
   // element count and the stride between columns, in elements
   const uint64_t elems = MODE == kRealPair ? n / 2 : n;
   const uint64_t col = MODE == kReal ? n : n / (MODE == kRealPair ? 2 : 1);
@@ -889,7 +891,8 @@ __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const d
       wb = v.y;
     }
     double sa = 0.0, sb = 0.0, la = 0.0, lb = 0.0, pa = 0.0, pb = 0.0;
-    for (int j0 = 0; j0 < m; j0 += CH) {
+    // from the last columns down: the overlaps' sweep left those in the L2
+    for (int j0 = (m - 1) / CH * CH; j0 >= 0; j0 -= CH) {
       double xa[CH], xb[CH];
 #pragma unroll
       for (int jj = 0; jj < CH; ++jj) {
@@ -975,6 +978,47 @@ __global__ void __launch_bounds__(128) orthogonalize_finish_kernel(const double*
   }
 }
 
+// The record of a queued step: norms before and after, the DGKS verdict and the last overlap.
+__global__ void __launch_bounds__(128) lanczos_record_kernel(const double* __restrict__ partials, int G, int m,
+                                                             const double* __restrict__ h, double* __restrict__ record) {
+  __shared__ double tree[2][128];
+  double b = 0.0, a = 0.0;
+  for (int k = threadIdx.x; k < G; k += 128) {
+    b += partials[2 * k];
+    a += partials[2 * k + 1];
+  }
+  tree[0][threadIdx.x] = b;
+  tree[1][threadIdx.x] = a;
+  __syncthreads();
+  for (int width = 64; width > 0; width >>= 1) {
+    if (threadIdx.x < width) {
+      tree[0][threadIdx.x] += tree[0][threadIdx.x + width];
+      tree[1][threadIdx.x] += tree[1][threadIdx.x + width];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    const double before = sqrt(fmax(tree[0][0], 0.0)), after = sqrt(fmax(tree[1][0], 0.0));
+    record[0] = before;
+    record[1] = after;
+    record[2] = before > 2.220446049250313e-16 && after <= 0.70710678118654752440 * before ? 1.0 : 0.0;
+    record[3] = isfinite(after) && after > 1.0e-14 ? 1.0 : 0.0;
+    record[FusedOrtho::kRecordHead + 2 * (m - 1)] = h[0];
+    record[FusedOrtho::kRecordHead + 2 * (m - 1) + 1] = h[1];
+  }
+}
+
+// dst = src / the record's norm
+__global__ void __launch_bounds__(kThreads) scale_by_record_kernel(const double* __restrict__ src,
+                                                                   double* __restrict__ dst, uint64_t count,
+                                                                   const double* __restrict__ record) {
+  if (record[3] == 0.0) return;
+  const double divisor = record[1];
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride)
+    dst[i] = src[i] / divisor;
+}
+
 }  // namespace
 
 uint64_t exclusive_scan_counts(const uint32_t* counts, uint64_t n, DeviceBuffer& row_ptr, bool* is64) {
@@ -1037,9 +1081,9 @@ double device_max_shifted_column(const double* diag, const double* offsum, uint6
   return m;
 }
 
-BlockOps::BlockOps(int device, cudaStream_t stream) : device_(device), stream_(stream) {
+BlockOps::BlockOps(int device, cudaStream_t stream)
+    : device_(device), stream_(stream), sms_(sm_count(device)), fused_(device, sms_) {
   QMBED_CUDA(cudaSetDevice(device_));
-  sms_ = sm_count(device_);
 }
 
 BlockOps::~BlockOps() {
@@ -1418,7 +1462,8 @@ void BlockOps::gram_schmidt_pass(const double* A, uint64_t n, int m, double beta
   const size_t smem = static_cast<size_t>(m) * 16;
   if (smem > 48 * 1024)
     QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, h, beta, three_term ? 1 : 0, w, w, partials_.as<double>());
+  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, h, beta, nullptr, three_term ? 1 : 0, w, w,
+                                               partials_.as<double>());
   QMBED_LAUNCH_CHECK();
   orthogonalize_finish_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, h + 2 * (m - 1),
                                                       results_.as<double>());
@@ -1428,6 +1473,35 @@ void BlockOps::gram_schmidt_pass(const double* A, uint64_t n, int m, double beta
   *before_sq = host_results_[0];
   *after_sq = host_results_[1];
   if (last_overlap) *last_overlap = C64(host_results_[2], host_results_[3]);
+}
+
+void BlockOps::lanczos_step(const double* A, uint64_t n, int m, double* w, double* slot, bool cplx) {
+  if (fused_.applies(n, m)) {
+    fused_.step(A, n, m, w, w, slot, cplx, true, stream_);
+    return;
+  }
+  const double* beta = nullptr;
+  double* record = fused_.next_record(m, &beta);
+  ensure_coeffs(static_cast<size_t>(m) * 16);
+  double* h = coeffs_.as<double>();
+  dots_device(A, n, m, w, n, 64, cplx, h);
+  const int G = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kOrthoThreads - 1) / kOrthoThreads,
+                                                                          4ull * sms_)));
+  ensure_partials(2 * static_cast<size_t>(G) + 64);
+  const int mode = cplx ? kComplex : (n % 2 == 0 ? kRealPair : kReal);
+  auto kernel = mode == kComplex ? orthogonalize_kernel<kComplex>
+                                 : (mode == kRealPair ? orthogonalize_kernel<kRealPair> : orthogonalize_kernel<kReal>);
+  const size_t smem = static_cast<size_t>(m) * 16;
+  if (smem > 48 * 1024)
+    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, h, 0.0, beta, 1, w, w, partials_.as<double>());
+  QMBED_LAUNCH_CHECK();
+  lanczos_record_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, m, h + 2 * (m - 1), record);
+  QMBED_LAUNCH_CHECK();
+  if (!slot) return;
+  const uint64_t count = n * (cplx ? 2 : 1);
+  scale_by_record_kernel<<<stream_grid(count, sms_), kThreads, 0, stream_>>>(w, slot, count, record);
+  QMBED_LAUNCH_CHECK();
 }
 
 void BlockOps::project_out(const double* A, uint64_t n, int m, const double* src, double* w, bool cplx, C64* h,
@@ -1445,7 +1519,7 @@ void BlockOps::project_out(const double* A, uint64_t n, int m, const double* src
   const size_t smem = static_cast<size_t>(m) * 16;
   if (smem > 48 * 1024)
     QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, hd, 0.0, 2, src, w, partials_.as<double>());
+  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, hd, 0.0, nullptr, 2, src, w, partials_.as<double>());
   QMBED_LAUNCH_CHECK();
   orthogonalize_finish_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, hd, results_.as<double>());
   QMBED_LAUNCH_CHECK();

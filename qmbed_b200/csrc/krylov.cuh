@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gram_schmidt.cuh"
 
 namespace qmbed {
 
@@ -53,6 +54,19 @@ class BlockOps {
   // host synchronisation.
   void project_out(const double* A, uint64_t n, int m, const double* src, double* w, bool cplx, C64* h,
                    double* src_norm_sq, double* out_norm_sq);
+  // Lanczos steps queued without a host round trip, up to `steps` of them on
+  // panels of at most m columns (`beta`: the norm before the first step). A
+  // step orthogonalises w against the m columns of A as gram_schmidt_pass does
+  // (three-term test) and writes w / |w| to `slot` (when given and |w| > 1e-14);
+  // lanczos_finish waits for the records. Vectors that the fused kernel serves
+  // get their DGKS second pass on the device; with larger ones a record whose
+  // `second` is set is short of it, and it and the steps after it are to be redone.
+  bool lanczos_fused(uint64_t n, int m) const { return fused_.applies(n, m); }
+  void lanczos_begin(int steps, int m, double beta) { fused_.begin(steps, m, beta, stream_); }
+  void lanczos_step(const double* A, uint64_t n, int m, double* w, double* slot, bool cplx);
+  void lanczos_finish(std::vector<OrthoRecord>& records) { fused_.finish(records, stream_); }
+  // One vector against m columns with the second pass, into slot (w when null).
+  FusedOrtho& fused() { return fused_; }
   double norm(const void* w, uint64_t n, int precision, bool cplx);
   // w = src - sum_j h_j A_j (src = w when null); returns ||w|| when `want_norm`.
   double subtract(const void* A, uint64_t ld, int m, const C64* h, void* w, uint64_t n, int precision, bool cplx,
@@ -89,6 +103,7 @@ class BlockOps {
   int device_;
   cudaStream_t stream_;
   int sms_ = 148;
+  FusedOrtho fused_;
   DeviceBuffer partials_, results_, coeffs_;
   std::vector<DeviceBuffer> workspace_;
   size_t partials_doubles_ = 0, coeffs_bytes_ = 0;

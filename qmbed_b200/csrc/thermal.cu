@@ -29,6 +29,7 @@ namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
 constexpr double kDgks = 0.70710678118654752440;  // 1/sqrt(2)
+constexpr int kQueuedSteps = 32;  // Lanczos steps queued before the host reads their records
 
 int grid_for(uint64_t n, int sms) {
   return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 8ull * sms)));
@@ -140,7 +141,41 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   d.second_passes = 0;
   std::vector<double> betas;
   double previous_beta = 0.0;
-  for (int index = 0; index < capacity; ++index) {
+  // Steps queue up to kQueuedSteps at a time (no host round trip between
+  // them); one that needs a second pass the queue does not make is redone by
+  // the loop below, which then goes on step by step to the next queue.
+  bool finished = false;
+  for (int index = 0; index < capacity && !finished; ++index) {
+    {
+      const int end = std::min(capacity, index + kQueuedSteps);
+      ops.lanczos_begin(end - index, end, previous_beta);
+      for (int i = index; i < end; ++i) {
+        op.apply(64, cplx, col(i), w.get());
+        ops.lanczos_step(d.basis.as<double>(), n, i + 1, w.as<double>(),
+                         i + 1 < capacity ? reinterpret_cast<double*>(col(i + 1)) : nullptr, cplx);
+      }
+      std::vector<OrthoRecord> records;
+      ops.lanczos_finish(records);
+      const bool whole = ops.lanczos_fused(n, end);
+      int i = index;
+      for (; i < end && !finished; ++i) {
+        const OrthoRecord& r = records[static_cast<size_t>(i - index)];
+        if (r.second && !whole) break;
+        ++d.applications;
+        if (std::fabs(r.h.back().imag()) > std::max(tolerance, 1.0e-10)) raise(QMBED_NON_HERMITIAN, "");
+        if (r.second) ++d.second_passes;
+        d.diagonal.push_back(r.h.back().real());
+        betas.push_back(r.norm);
+        previous_beta = r.norm;
+        finished = i + 1 == capacity || !(r.norm > tolerance);
+      }
+      index = i;
+      if (finished) break;
+      if (i == end) {
+        --index;  // the next queue starts here
+        continue;
+      }
+    }
     op.apply(64, cplx, col(index), w.get());
     ++d.applications;
     // alpha = <q_index, w> is the last overlap of the pass; the pass also
