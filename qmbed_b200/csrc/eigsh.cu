@@ -39,6 +39,8 @@ constexpr double kMixedHandover = 2.0e-6;
 
 struct Panel {
   DeviceBuffer buf;
+  Scratch kept;
+  void* base = nullptr;
   uint64_t n = 0;
   int cols = 0;
   int prec = 64;
@@ -50,8 +52,18 @@ struct Panel {
     prec = prec_;
     cplx = cplx_;
     buf.allocate(std::max<size_t>(1, static_cast<size_t>(n) * cols * es()));
+    base = buf.get();
   }
-  void* col(int j) const { return static_cast<char*>(buf.get()) + static_cast<size_t>(j) * n * es(); }
+  // in a workspace slot of the handle
+  void alloc(uint64_t n_, int cols_, int prec_, bool cplx_, BlockOps& ops, int slot) {
+    n = n_;
+    cols = cols_;
+    prec = prec_;
+    cplx = cplx_;
+    kept.take(ops, slot, static_cast<size_t>(n) * cols * es());
+    base = kept.get();
+  }
+  void* col(int j) const { return static_cast<char*>(base) + static_cast<size_t>(j) * n * es(); }
 };
 
 struct Ctx {
@@ -245,9 +257,9 @@ EigshResult lanczos_window(Ctx& c, const EigshOptions& o, const void* initial_de
   const size_t krylov = std::min({requested, o.max_iterations, static_cast<size_t>(n)});
   if (krylov <= o.eigenpairs) raise(QMBED_INVALID_OPTIONS, "the effective Krylov dimension must exceed eigenpairs");
   Panel V;
-  V.alloc(n, static_cast<int>(krylov), c.prec, c.cplx);
+  V.alloc(n, static_cast<int>(krylov), c.prec, c.cplx, c.ops, 19);
   Panel work;
-  work.alloc(n, 1, c.prec, c.cplx);
+  work.alloc(n, 1, c.prec, c.cplx, c.ops, 20);
   void* out = work.col(0);
   if (initial_device) {
     c.copy(initial_device, V.col(0));
@@ -406,14 +418,14 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
   auto keep_for = [&](int active) { return std::max(std::min(std::max(active, wider), m / 2), 1); };
   const int keep_cap = keep_for(k);  // candidates per cycle never exceed this
   Panel Q, W, C, CA, RC, RCA, work;
-  Q.alloc(n, k + m, c.prec, c.cplx);  // [locked | basis]
-  W.alloc(n, m, c.prec, c.cplx);      // applied actions of the basis
-  C.alloc(n, keep_cap, c.prec, c.cplx);   // Ritz candidates of this cycle
-  CA.alloc(n, keep_cap, c.prec, c.cplx);  // their actions
+  Q.alloc(n, k + m, c.prec, c.cplx, c.ops, 12);  // [locked | basis]
+  W.alloc(n, m, c.prec, c.cplx, c.ops, 13);      // applied actions of the basis
+  C.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 14);   // Ritz candidates of this cycle
+  CA.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 15);  // their actions
   const int retain_cap = std::max(keep_cap, n_initial);
-  RC.alloc(n, retain_cap, c.prec, c.cplx);   // vectors retained for the next cycle
-  RCA.alloc(n, retain_cap, c.prec, c.cplx);  // their actions
-  work.alloc(n, 1, c.prec, c.cplx);
+  RC.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 16);   // vectors retained for the next cycle
+  RCA.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 17);  // their actions
+  work.alloc(n, 1, c.prec, c.cplx, c.ops, 18);
   void* tmp = work.col(0);
   std::vector<double> locked_values, locked_residuals;
   int l = 0;

@@ -95,9 +95,9 @@ class KrylovExp {
  public:
   KrylovExp(const LinearOperatorView& op, BlockOps& ops, size_t krylov)
       : op_(op), ops_(ops), n_(op.dim), m_(static_cast<int>(std::max<uint64_t>(std::min<uint64_t>(krylov, op.dim), 1))) {
-    panel_.allocate(static_cast<size_t>(m_) * n_ * 16);
-    w_.allocate(std::max<uint64_t>(n_, 1) * 16);
-    coeff_.allocate(static_cast<size_t>(2 * m_) * sizeof(double));
+    panel_.take(ops, 32, static_cast<size_t>(m_) * n_ * 16);
+    w_.take(ops, 33, n_ * 16);
+    coeff_.take(ops, 34, static_cast<size_t>(2 * m_) * sizeof(double));
   }
 
   // lanczos_projection(_real) (src/solve/mod.rs:2909-3054) of a device state
@@ -181,7 +181,7 @@ class KrylovExp {
   BlockOps& ops_;
   uint64_t n_;
   int m_;
-  DeviceBuffer panel_, w_, coeff_;
+  Scratch panel_, w_, coeff_;
 };
 
 bool host_vector_is_real(const double* v, uint64_t n) {
@@ -220,7 +220,7 @@ void evolve(const LinearOperatorView& op, const double* initial, const Evolution
   const uint64_t n = op.dim;
   const cudaStream_t s = ops.stream();
   KrylovExp krylov(op, ops, o.krylov_dimension);
-  DeviceBuffer a(std::max<uint64_t>(n, 1) * 16), b(std::max<uint64_t>(n, 1) * 16);
+  Scratch a(ops, 35, n * 16), b(ops, 36, n * 16);
   double* current = a.as<double>();
   double* candidate = b.as<double>();
   QMBED_CUDA(cudaMemcpyAsync(current, initial, n * 16, cudaMemcpyHostToDevice, s));

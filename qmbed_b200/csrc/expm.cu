@@ -146,7 +146,7 @@ size_t expm_apply(const ExpmPlan& plan, const LinearOperatorView& op, void* stat
   cudaStream_t stream = ops.stream();
   const int grid = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kThreads - 1) / kThreads,
                                                                              4ULL * ops.sms())));
-  DeviceBuffer partials(2 * grid * sizeof(double));
+  Scratch partials(ops, 28, 2 * grid * sizeof(double));
   std::vector<double> host(2 * grid);
   auto read_max = [&](int stride_, int offset) {
     QMBED_CUDA(cudaMemcpyAsync(host.data(), partials.get(), 2 * grid * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -167,23 +167,25 @@ size_t expm_apply(const ExpmPlan& plan, const LinearOperatorView& op, void* stat
   const C64 eta = std::exp(factor * plan.shift);
   if (!std::isfinite(eta.real()) || !std::isfinite(eta.imag()))
     raise(QMBED_UNSUPPORTED_BACKEND, "exponential action overflowed its scalar trace shift");
-  DeviceBuffer term(bytes), applied(bytes), sum(bytes);
+  Scratch term_buf(ops, 29, bytes), applied_buf(ops, 30, bytes), sum(ops, 31, bytes);
+  void* term = term_buf.get();
+  void* applied = applied_buf.get();
   size_t applications = 0;
   for (size_t s = 0; s < plan.scaling; ++s) {
-    ops.copy(state, term.get(), bytes);
+    ops.copy(state, term, bytes);
     ops.copy(state, sum.get(), bytes);
-    double previous = inf_norm(term.get());
+    double previous = inf_norm(term);
     for (size_t order = 1; order <= plan.degree; ++order) {
-      op.apply(precision, true, term.get(), applied.get());
+      op.apply(precision, true, term, applied);
       ++applications;
       const C64 scale = factor / static_cast<double>(order);
       if (precision == 64)
-        taylor_update_kernel<double><<<grid, kThreads, 0, stream>>>(n, applied.as<double>(), term.as<double>(),
+        taylor_update_kernel<double><<<grid, kThreads, 0, stream>>>(n, static_cast<double*>(applied), static_cast<const double*>(term),
                                                                     sum.as<double>(), scale.real(), scale.imag(),
                                                                     plan.shift.real(), plan.shift.imag(),
                                                                     partials.as<double>());
       else
-        taylor_update_kernel<float><<<grid, kThreads, 0, stream>>>(n, applied.as<float>(), term.as<float>(),
+        taylor_update_kernel<float><<<grid, kThreads, 0, stream>>>(n, static_cast<float*>(applied), static_cast<const float*>(term),
                                                                    sum.as<float>(), scale.real(), scale.imag(),
                                                                    plan.shift.real(), plan.shift.imag(),
                                                                    partials.as<double>());

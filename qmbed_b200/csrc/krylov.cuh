@@ -111,6 +111,37 @@ class BlockOps {
   size_t host_results_doubles_ = 0;
 };
 
+// Work buffer of one call: a workspace slot of the handle while it is at most
+// kKeptBytes (kept for the next call on the handle and freed with it; the
+// driver takes 0.1 to 5 ms per allocation and free), else an allocation of the
+// call's own. Slots: 0-9 filtered solver, 10 projected eigenproblems, 12-18
+// thick restart, 19-20 Lanczos window, 21-23 thermal Lanczos, 24-27 Chebyshev
+// propagator, 28-31 Taylor action, 32-36 Krylov evolution.
+class Scratch {
+ public:
+  static constexpr size_t kKeptBytes = 1ull << 30;
+  Scratch() = default;
+  Scratch(BlockOps& ops, int slot, size_t bytes) { take(ops, slot, bytes); }
+  void take(BlockOps& ops, int slot, size_t bytes) {
+    bytes = bytes > 0 ? bytes : 1;
+    if (bytes <= kKeptBytes) {
+      ptr_ = ops.workspace(slot, bytes);
+    } else {
+      own_.allocate(bytes);
+      ptr_ = own_.get();
+    }
+  }
+  void* get() const { return ptr_; }
+  template <typename T>
+  T* as() const {
+    return static_cast<T*>(ptr_);
+  }
+
+ private:
+  DeviceBuffer own_;
+  void* ptr_ = nullptr;
+};
+
 // Symmetric tridiagonal eigenproblem on the host by implicit QL with
 // Wilkinson shifts: ascending values; V row-major n x n (V[row * n + col],
 // column col belongs to values[col]), or only its first row when first_row.

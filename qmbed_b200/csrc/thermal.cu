@@ -113,12 +113,12 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   if (wanted > 8192) raise(QMBED_UNSUPPORTED_BACKEND, "Krylov dimensions above 8192 are not supported");
   const int capacity = static_cast<int>(wanted);
   const size_t panel_bytes = static_cast<size_t>(capacity) * n * width;
-  if (d.basis.bytes() < panel_bytes) d.basis.allocate(panel_bytes);  // kept across repeated runs
-  DeviceBuffer w(n * width);
-  auto col = [&](int j) { return static_cast<char*>(d.basis.get()) + static_cast<size_t>(j) * n * width; };
+  if (!d.lent && d.basis.bytes() < panel_bytes) d.basis.allocate(panel_bytes);  // kept across repeated runs
+  Scratch w(ops, 21, n * width);
+  auto col = [&](int j) { return static_cast<char*>(d.panel()) + static_cast<size_t>(j) * n * width; };
   // one Gram-Schmidt pass over q_0 .. q_{m-1}; returns (|w'|^2, |w''|^2, alpha)
   auto pass = [&](int m, double beta, bool three_term, double* before_sq, double* after_sq, C64* alpha) {
-    ops.gram_schmidt_pass(d.basis.as<double>(), n, m, beta, three_term, w.as<double>(), cplx, before_sq, after_sq,
+    ops.gram_schmidt_pass(static_cast<double*>(d.panel()), n, m, beta, three_term, w.as<double>(), cplx, before_sq, after_sq,
                           alpha);
   };
 
@@ -151,7 +151,7 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
       ops.lanczos_begin(end - index, end, previous_beta);
       for (int i = index; i < end; ++i) {
         op.apply(64, cplx, col(i), w.get());
-        ops.lanczos_step(d.basis.as<double>(), n, i + 1, w.as<double>(),
+        ops.lanczos_step(static_cast<double*>(d.panel()), n, i + 1, w.as<double>(),
                          i + 1 < capacity ? reinterpret_cast<double*>(col(i + 1)) : nullptr, cplx);
       }
       std::vector<OrthoRecord> records;
@@ -265,13 +265,13 @@ std::vector<C64> project_observable(const LanczosDecomposition& d, const LinearO
     DeviceBuffer applied(n * 16);
     for (int input = 0; input < (ltlm ? m : 1); ++input) {
       a.apply(64, true, d.column(input), applied.get());
-      ops.dots(d.basis.get(), n, m, applied.get(), n, 64, true, out.data() + static_cast<size_t>(input) * m);
+      ops.dots(d.panel(), n, m, applied.get(), n, 64, true, out.data() + static_cast<size_t>(input) * m);
     }
   } else if (a.real) {
     DeviceBuffer applied(n * 8);
     for (int input = 0; input < (ltlm ? m : 1); ++input) {
       a.apply(64, false, d.column(input), applied.get());
-      ops.dots(d.basis.get(), n, m, applied.get(), n, 64, false, out.data() + static_cast<size_t>(input) * m);
+      ops.dots(d.panel(), n, m, applied.get(), n, 64, false, out.data() + static_cast<size_t>(input) * m);
     }
   } else {
     // complex observable on a real basis: widen the input column, split the
@@ -285,8 +285,8 @@ std::vector<C64> project_observable(const LanczosDecomposition& d, const LinearO
       a.apply(64, true, wide.get(), applied.get());
       split_complex_kernel<<<G, 256, 0, ops.stream()>>>(applied.as<double>(), re, im, n);
       QMBED_LAUNCH_CHECK();
-      ops.dots(d.basis.get(), n, m, re, n, 64, false, ore.data());
-      ops.dots(d.basis.get(), n, m, im, n, 64, false, oim.data());
+      ops.dots(d.panel(), n, m, re, n, 64, false, ore.data());
+      ops.dots(d.panel(), n, m, im, n, 64, false, oim.data());
       for (int j = 0; j < m; ++j) out[static_cast<size_t>(input) * m + j] = C64(ore[j].real(), oim[j].real());
     }
   }
@@ -392,12 +392,12 @@ void lanczos_combine(const LanczosDecomposition& d, const std::vector<C64>& c, d
     DeviceBuffer coeff(c.size() * 16);
     QMBED_CUDA(cudaMemcpyAsync(coeff.get(), c.data(), c.size() * 16, cudaMemcpyHostToDevice, s));
     const int G = grid_for(d.n, ops.sms());
-    real_panel_combine_kernel<<<G, 256, 2 * c.size() * sizeof(double), s>>>(d.basis.as<double>(), d.n, d.size,
+    real_panel_combine_kernel<<<G, 256, 2 * c.size() * sizeof(double), s>>>(static_cast<double*>(d.panel()), d.n, d.size,
                                                                              coeff.as<double>(), out);
     QMBED_LAUNCH_CHECK();
     ops.sync();
   } else {
-    ops.combine(d.basis.get(), d.n, d.size, c.data(), 1, out, d.n, d.n, 64, true);
+    ops.combine(d.panel(), d.n, d.size, c.data(), 1, out, d.n, d.n, 64, true);
     ops.sync();
   }
 }
@@ -432,11 +432,13 @@ void ftlm_sample(const LinearOperatorView& op, int vectors, uint64_t seed, size_
   if (!ok) raise(QMBED_INVALID_OPTIONS, "inverse temperatures must be nonempty, finite, and nonnegative");
   const uint64_t n = op.dim;
   const bool cplx = !op.real;
-  DeviceBuffer start(std::max<uint64_t>(n, 1) * (cplx ? 16 : 8));
+  Scratch start(ops, 22, n * (cplx ? 16 : 8));
   log_partition.clear();
   mean_energy.clear();
   lengths.clear();
   LanczosDecomposition d;
+  const Scratch basis(ops, 23, std::min<uint64_t>(std::min<uint64_t>(krylov, n), 8192) * n * (cplx ? 16 : 8));
+  d.lent = basis.get();
   for (int r = 0; r < vectors; ++r) {
     ftlm_start_vector(op, seed, r, start.as<double>(), ops);
     lanczos_ritz_device(op, start.as<double>(), cplx, krylov, tolerance, d, ops, false);

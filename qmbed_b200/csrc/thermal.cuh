@@ -23,13 +23,15 @@ struct LanczosDecomposition {
   int size = 0;
   double initial_norm = 0.0;
   DeviceBuffer basis;
+  void* lent = nullptr;  // the basis in a buffer of the caller instead
+  void* panel() const { return lent ? lent : basis.get(); }
   std::vector<double> diagonal, off_diagonal;
   std::vector<double> eigenvalues, V;
   size_t applications = 0;
   int second_passes = 0;     // DGKS second Gram-Schmidt passes
   bool full_vectors = true;  // V holds every row (else the first row only)
   const void* column(int j) const {
-    return static_cast<const char*>(basis.get()) + static_cast<size_t>(j) * n * (real ? 8 : 16);
+    return static_cast<const char*>(panel()) + static_cast<size_t>(j) * n * (real ? 8 : 16);
   }
   double vec(int row, int col) const { return V[static_cast<size_t>(row) * size + col]; }
 };
