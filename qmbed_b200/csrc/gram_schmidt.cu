@@ -19,10 +19,9 @@ constexpr int kMaxColumns = 512;
 constexpr unsigned kSpinLimit = 1u << 22;
 constexpr double kEps = 2.220446049250313e-16;
 constexpr double kDgks = 0.70710678118654752440;  // 1/sqrt(2)
-constexpr int kRecordHead = FusedOrtho::kRecordHead;  // before, norm, second, ok; then 2 m overlaps
+constexpr int kRecordHead = FusedOrtho::kRecordHead;  // before, norm, second, ok, four barrier counters; then 2 m overlaps
 
 struct GridState {
-  unsigned count, generation;
   int status, pad;
   double first[kRecordHead];  // what a record before the first would hold
 };
@@ -35,10 +34,10 @@ struct OrthoArgs {
   double* w;
   double* slot;
   int three_term;
-  const double* beta;  // previous record's norm
+  const double* beta;  // previous record's norm, followed by its `second`
   double* record;
-  double* partials;    // [m][G][1 or 2], then [G][2]
-  GridState* grid;
+  double* partials;    // for each pass [m][G][1 or 2], then [G][2]
+  int* status;
 };
 
 __device__ __forceinline__ double warp_total(double v) {
@@ -47,36 +46,63 @@ __device__ __forceinline__ double warp_total(double v) {
   return v;
 }
 
-// Barrier of the whole (cooperative) grid with a bounded wait; false when a
-// block gave up, after which every block leaves.
-__device__ bool grid_barrier(GridState* g, unsigned blocks) {
+// Barrier of the whole (cooperative) grid on a counter of its own, with a
+// bounded wait; false when a block gave up, after which every block leaves.
+__device__ bool grid_barrier(unsigned* counter, int* status, unsigned blocks) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile GridState* v = g;
-    ok = v->status == 0;
-    if (ok) {
-      const unsigned generation = v->generation;
-      __threadfence();
-      if (atomicAdd(&g->count, 1u) == blocks - 1) {
-        v->count = 0;
-        __threadfence();
-        atomicAdd(&g->generation, 1u);
-      } else {
-        unsigned polls = 0;
-        while (v->generation == generation) {
-          if (++polls > kSpinLimit || v->status != 0) {
-            atomicExch(&g->status, 1);
-            ok = 0;
-            break;
-          }
-        }
+    ok = 1;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    unsigned polls = 0, seen;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+      if (seen < blocks && ++polls > kSpinLimit) {
+        atomicExch(status, 1);
+        ok = 0;
       }
-      __threadfence();
-    }
+    } while (seen < blocks && ok);
   }
   __syncthreads();
   return ok != 0;
+}
+
+// Overlaps of the slab's vector with the panel's columns, one warp per column
+// (two at once: their reads are in flight together), to this block's partials.
+template <bool CPLX>
+__device__ __forceinline__ void slab_overlaps(const OrthoArgs& a, const double* ws, uint64_t r0, int rows,
+                                              double* partials) {
+  constexpr int W = CPLX ? 2 : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j = warp; j < a.m; j += 2 * kWarps) {
+    const bool pair = j + kWarps < a.m;
+    const double* q = a.A + (static_cast<uint64_t>(j) * a.n + r0) * W;
+    const double* p = q + (pair ? static_cast<uint64_t>(kWarps) * a.n * W : 0);
+    double sum[2][2] = {};
+#pragma unroll 4
+    for (int r = lane; r < rows; r += 32) {
+      if (CPLX) {
+        const double2 y = reinterpret_cast<const double2*>(ws)[r];
+        const double2 x = reinterpret_cast<const double2*>(q)[r], z = reinterpret_cast<const double2*>(p)[r];
+        sum[0][0] += x.x * y.x + x.y * y.y;
+        sum[0][1] += x.x * y.y - x.y * y.x;
+        sum[1][0] += z.x * y.x + z.y * y.y;
+        sum[1][1] += z.x * y.y - z.y * y.x;
+      } else {
+        sum[0][0] += q[r] * ws[r];
+        sum[1][0] += p[r] * ws[r];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double sr = warp_total(sum[h][0]), si = CPLX ? warp_total(sum[h][1]) : 0.0;
+      if (lane == 0 && (h == 0 || pair)) {
+        double* to = partials + (static_cast<size_t>(j + h * kWarps) * gridDim.x + blockIdx.x) * W;
+        to[0] = sr;
+        if (CPLX) to[1] = si;
+      }
+    }
+  }
 }
 
 // A block owns `rows` consecutive rows; its part of the vector stays in shared
@@ -86,11 +112,19 @@ __device__ bool grid_barrier(GridState* g, unsigned blocks) {
 // same overlaps without a second launch). Subtraction: thread groups share a
 // row's columns when the slab has fewer rows than the block threads.
 //
-// Latency-bound by its two barriers per pass and the panel reads between them
-// (the panels it serves fit the L2; keeping a block's slab of the panel in
-// shared memory changed nothing). Measured (B200) at 9252 rows and up to 44
-// columns: 20 us with its second pass, on the device's own time, against nine
-// launches (16 us of kernels) and two host round trips, about 100 us a step.
+// When the step before made a second pass, this one most likely does: the
+// second pass's overlaps are then taken along with the first one's norms, in
+// front of the same barrier (and left unused if the test says otherwise; the
+// results do not depend on it).
+//
+// Latency-bound by the barriers, the panel reads between them and the sums of
+// the partials (the panels it serves fit the L2; keeping a block's slab of the
+// panel in shared memory changed nothing). Measured (B200) at 9252 rows and up
+// to 44 columns with the second pass: 15.5 us on
+// the device's own time, 19.9 us with the second pass behind barriers of its
+// own, an arrival count that the last block resets and one column at a time; as
+// nine launches (16 us of kernels) and two host round trips about 100 us a step.
+// Slabs of 64 rows 17.2 us, of 256 15.6; 1024 threads 17.2.
 template <bool CPLX>
 __global__ void __launch_bounds__(kThreads, 1) ortho_fused_kernel(const __grid_constant__ OrthoArgs a) {
   constexpr int W = CPLX ? 2 : 1;
@@ -104,50 +138,45 @@ __global__ void __launch_bounds__(kThreads, 1) ortho_fused_kernel(const __grid_c
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * a.rows;
   const int rows = static_cast<int>(min(static_cast<uint64_t>(a.rows), a.n - r0));
-  double* norms = a.partials + static_cast<size_t>(a.m) * G * W;
+  const size_t pass_size = static_cast<size_t>(a.m) * G * W + 2 * static_cast<size_t>(G);
+  unsigned* counters = reinterpret_cast<unsigned*>(a.record + 4);
+  const bool ahead = __ldcg(a.beta + 1) != 0.0;
+  if (__ldcg(a.status) != 0) return;  // a step before this one gave up
   for (int t = threadIdx.x; t < rows * W; t += kThreads) ws[t] = a.src[r0 * W + t];
   __syncthreads();
   double before = 0.0, after = 0.0;
   bool second = false;
   for (int pass = 0; pass < 2; ++pass) {
-    for (int j = warp; j < a.m; j += kWarps) {
-      const double* q = a.A + (static_cast<uint64_t>(j) * a.n + r0) * W;
-      double sr = 0.0, si = 0.0;
-#pragma unroll 4
-      for (int r = lane; r < rows; r += 32) {
-        if (CPLX) {
-          const double2 x = reinterpret_cast<const double2*>(q)[r];
-          const double2 y = reinterpret_cast<const double2*>(ws)[r];
-          sr += x.x * y.x + x.y * y.y;
-          si += x.x * y.y - x.y * y.x;
-        } else {
-          sr += q[r] * ws[r];
+    double* partials = a.partials + pass * pass_size;
+    double* norms = partials + pass_size - 2 * static_cast<size_t>(G);
+    if (pass == 0 || !ahead) {
+      slab_overlaps<CPLX>(a, ws, r0, rows, partials);
+      if (!grid_barrier(counters + 2 * pass, a.status, G)) return;
+    }
+    // four columns of a warp at once
+    for (int j0 = warp; j0 < a.m; j0 += 4 * kWarps) {
+      double sum[4][W] = {};
+#pragma unroll 2
+      for (unsigned b = lane; b < G; b += 32) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (j0 + h * kWarps < a.m) {
+            const double* p = partials + (static_cast<size_t>(j0 + h * kWarps) * G + b) * W;
+#pragma unroll
+            for (int c = 0; c < W; ++c) sum[h][c] += __ldcg(p + c);
+          }
         }
       }
-      sr = warp_total(sr);
-      if (CPLX) si = warp_total(si);
-      if (lane == 0) {
-        double* p = a.partials + (static_cast<size_t>(j) * G + blockIdx.x) * W;
-        p[0] = sr;
-        if (CPLX) p[1] = si;
-      }
-    }
-    if (!grid_barrier(a.grid, G)) return;
-    for (int j = warp; j < a.m; j += kWarps) {
-      const double* p = a.partials + static_cast<size_t>(j) * G * W;
-      double sr = 0.0, si = 0.0;
-      for (unsigned b = lane; b < G; b += 32) {
-        sr += __ldcg(p + b * W);
-        if (CPLX) si += __ldcg(p + b * W + 1);
-      }
-      sr = warp_total(sr);
-      if (CPLX) si = warp_total(si);
-      if (lane == 0) {
-        hs[j * W] = sr;
-        if (CPLX) hs[j * W + 1] = si;
-        if (pass == 0 && blockIdx.x == 0) {
-          a.record[kRecordHead + 2 * j] = sr;
-          a.record[kRecordHead + 2 * j + 1] = CPLX ? si : 0.0;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int j = j0 + h * kWarps;
+#pragma unroll
+        for (int c = 0; c < W; ++c) {
+          const double v = warp_total(sum[h][c]);
+          if (lane == 0 && j < a.m) {
+            hs[j * W + c] = v;
+            if (pass == 0 && blockIdx.x == 0) a.record[kRecordHead + 2 * j + c] = v;
+          }
         }
       }
     }
@@ -222,9 +251,11 @@ __global__ void __launch_bounds__(kThreads, 1) ortho_fused_kernel(const __grid_c
       for (int q = 0; q < kWarps; ++q) s += red[q][threadIdx.x];
       norms[2 * blockIdx.x + threadIdx.x] = s;
     }
-    if (!grid_barrier(a.grid, G)) return;
+    if (pass == 0 && ahead) slab_overlaps<CPLX>(a, ws, r0, rows, partials + pass_size);
+    if (!grid_barrier(counters + 2 * pass + 1, a.status, G)) return;
     if (warp < 2) {
       double s = 0.0;
+#pragma unroll 4
       for (unsigned b = lane; b < G; b += 32) s += __ldcg(norms + 2 * b + warp);
       s = warp_total(s);
       if (lane == 0) total[warp] = s;
@@ -275,7 +306,7 @@ void FusedOrtho::begin(int steps, int m, double beta, cudaStream_t stream) {
   count_ = 0;
   columns_.clear();
   const size_t bytes = sizeof(GridState) + static_cast<size_t>(steps) * cap_ * sizeof(double);
-  const size_t part = (static_cast<size_t>(m) * 2 + 2) * sms_ * sizeof(double);
+  const size_t part = 2 * (static_cast<size_t>(m) * 2 + 2) * sms_ * sizeof(double);
   if (state_.bytes() < bytes || partials_.bytes() < part) {
     QMBED_CUDA(cudaStreamSynchronize(stream));
     if (state_.bytes() < bytes) state_.allocate(bytes);
@@ -291,6 +322,7 @@ void FusedOrtho::begin(int steps, int m, double beta, cudaStream_t stream) {
   head.first[1] = beta;
   std::memcpy(host_, &head, sizeof head);
   QMBED_CUDA(cudaMemcpyAsync(state_.get(), host_, sizeof head, cudaMemcpyHostToDevice, stream));
+  QMBED_CUDA(cudaMemsetAsync(state_.as<GridState>() + 1, 0, bytes - sizeof head, stream));  // the barriers' counters
 }
 
 double* FusedOrtho::next_record(int m, const double** previous_norm) {
@@ -318,7 +350,7 @@ void FusedOrtho::step(const double* A, uint64_t n, int m, const double* src, dou
   a.three_term = three_term ? 1 : 0;
   a.record = next_record(m, &a.beta);
   a.partials = partials_.as<double>();
-  a.grid = state_.as<GridState>();
+  a.status = &state_.as<GridState>()->status;
   const unsigned grid = static_cast<unsigned>((n + a.rows - 1) / a.rows);
   const size_t smem = smem_bytes(a.rows, m, cplx);
   const void* kernel = cplx ? reinterpret_cast<const void*>(ortho_fused_kernel<true>)

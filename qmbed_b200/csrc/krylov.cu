@@ -630,14 +630,17 @@ __global__ void __launch_bounds__(1024) jacobi_kernel(int np, double* __restrict
 // lower part's size n padded to even np). A round rotates np/2 disjoint pairs
 // at once; J^H A J splits into the (np/2)^2 independent 2 x 2 blocks (pair s
 // rows, pair t columns), so rows and columns are rotated by one thread per
-// block in one pass, with two barriers per round (angles; blocks and vectors)
-// instead of five. What bounds it is the round's latency chain (shared reads,
+// block in one pass. What bounds it is the round's latency chain (shared reads,
 // one division and two square roots per angle, two barriers), not arithmetic:
-// the projected matrices are 8 to 40 wide. Measured (B200): 16 x 16 real 45 us
-// against 210 us and 40 x 40 real 303 us against 2268 us
-// for jacobi_kernel, which keeps both matrices in global memory as complex
-// numbers; that kernel remains for matrices beyond the shared memory.
-constexpr int kJacobiMaxThreads = 512;
+// the projected matrices are 8 to 44 wide. So the warps behind the first one or
+// two rotate the vectors while those compute the next round's angles, and the
+// angles lie as (c, s) pairs, which a warp reads without bank conflicts.
+// Measured (B200): 16 x 16 real 44 us and 44 x 44 real 234 us; 46 and 310 with
+// angles, then blocks and vectors; 210 us and (40 x 40) 2268 us for
+// jacobi_kernel, which keeps both matrices in global memory as complex numbers;
+// that kernel remains for matrices beyond the shared memory.
+constexpr int kJacobiBlockItems = 512;       // 2 x 2 blocks of a trip
+constexpr int kJacobiMaxThreads = 512 + 64;  // and up to two warps for the next round's angles
 constexpr size_t kJacobiMaxSmem = 200 * 1024;  // real n <= 112, complex n <= 78
 constexpr int kEigenWorkspace = 10;             // workspace slot of the handle (0-9: the filtered solver's)
 
@@ -676,7 +679,7 @@ __device__ __forceinline__ void jacobi_set(double2& v, double re) { v = make_dou
 
 size_t jacobi_smem_bytes(int n, bool cplx) {
   const size_t np = static_cast<size_t>(n + (n & 1));
-  return 2 * np * (np + 1) * (cplx ? 16 : 8) + (np / 2) * 4 * sizeof(double);
+  return 2 * np * (np + 1) * (cplx ? 16 : 8) + 2 * (np / 2) * ((cplx ? 2 : 1) * sizeof(double2) + sizeof(int));
 }
 
 // in: n x n row-major; values: n; vectors: column-major n x n.
@@ -692,7 +695,10 @@ __global__ void __launch_bounds__(kJacobiMaxThreads)
   const int np = n + (n & 1), half = np / 2, ld = np + 1;
   E* A = reinterpret_cast<E*>(jacobi_raw);
   E* V = A + np * ld;  // V[k * ld + j]: component k of vector j
-  double* rot = reinterpret_cast<double*>(V + np * ld);  // per pair: c, s, phase
+  // of this round and the next, per pair: (c, s), phase, (p, q)
+  constexpr int RW = CPLX ? 2 : 1;
+  double2* rot = reinterpret_cast<double2*>(V + np * ld);
+  int* pairs = reinterpret_cast<int*>(rot + 2 * RW * half);
   const double floor_rel = (2.220446049250313e-16 * np) * (2.220446049250313e-16 * np) * 1e-2;
   if (threadIdx.x == 0) previous_off = -1.0;
   for (int idx = threadIdx.x; idx < np * np; idx += blockDim.x) {
@@ -704,9 +710,48 @@ __global__ void __launch_bounds__(kJacobiMaxThreads)
     jacobi_set(V[i * ld + j], i == j ? 1.0 : 0.0);
   }
   __syncthreads();
-  // this thread's first block (s0, t0) and the step to its next one
-  const int s0 = threadIdx.x / half, t0 = threadIdx.x % half;
-  const int ds = blockDim.x / half, dt = blockDim.x % half;
+  // this thread's first block (s0, t0) of A and the step to its next one; the
+  // same for V, which the warps behind the angles' have
+  const int chain = (half + 31) / 32 * 32;
+  const int va = static_cast<int>(threadIdx.x) - chain, vn = static_cast<int>(blockDim.x) - chain;
+  const int s0 = threadIdx.x / half, t0 = threadIdx.x % half, ds = blockDim.x / half, dt = blockDim.x % half;
+  const int i0 = va >= 0 ? va / half : half, j0 = va >= 0 ? va % half : 0, di = vn / half, dj = vn % half;
+  // The rotations of a round, from A as the round before left it.
+  auto angles = [&](int round) {
+    const int t = threadIdx.x;
+    if (t >= half) return;
+    // round-robin pairing: position 0 is fixed, the others move by one place per round
+    int p = t == 0 ? 0 : t - round, q = np - 1 - t - round;
+    if (t != 0 && p < 1) p += np - 1;
+    if (q < 1) q += np - 1;
+    if (p > q) {
+      const int swap = p;
+      p = q;
+      q = swap;
+    }
+    const E b = A[p * ld + q];
+    const double mag = CPLX ? sqrt(jacobi_sq(b)) : fabs(jacobi_re(b));
+    double c = 1.0, s = 0.0, fr = 1.0, fi = 0.0;
+    if (mag != 0.0) {
+      // tan = 2 |b| / (d +- sqrt(d^2 + 4 |b|^2)), d = a_qq - a_pp: one square root, one
+      // division and one reciprocal square root in the round's dependent chain
+      const double d = jacobi_re(A[q * ld + q]) - jacobi_re(A[p * ld + p]), b2 = 2.0 * mag;
+      const double r = fabs(d) + sqrt(d * d + b2 * b2);
+      const double tt = r > 0.0 ? copysign(b2 / r, d) : 1.0;
+      c = rsqrt(tt * tt + 1.0);
+      s = tt * c;
+      if constexpr (CPLX) {
+        fr = b.x / mag;
+        fi = b.y / mag;
+      } else if (b < 0.0) {
+        s = -s;
+      }
+    }
+    const int at = (round & 1) * half + t;
+    rot[at] = make_double2(c, s);
+    if constexpr (CPLX) rot[2 * half + at] = make_double2(fr, fi);
+    pairs[at] = p | q << 16;
+  };
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     double off = 0.0, total = 0.0;
     for (int idx = threadIdx.x; idx < np * np; idx += blockDim.x) {
@@ -735,81 +780,56 @@ __global__ void __launch_bounds__(kJacobiMaxThreads)
     }
     __syncthreads();
     if (done) break;
+    angles(0);
+    __syncthreads();
     for (int round = 0; round < np - 1; ++round) {
-      // round-robin pairing: position 0 is fixed, the others move by one place per round
-      auto pair_of = [&](int t, int& p, int& q) {
-        int a = t == 0 ? 0 : t - round, b = np - 1 - t - round;
-        if (t != 0 && a < 1) a += np - 1;
-        if (b < 1) b += np - 1;
-        p = min(a, b);
-        q = max(a, b);
-      };
-      for (int t = threadIdx.x; t < half; t += blockDim.x) {
-        int p, q;
-        pair_of(t, p, q);
-        const E b = A[p * ld + q];
-        const double mag = CPLX ? sqrt(jacobi_sq(b)) : fabs(jacobi_re(b));
-        double c = 1.0, s = 0.0, fr = 1.0, fi = 0.0;
-        if (mag != 0.0) {
-          // tan = 2 |b| / (d +- sqrt(d^2 + 4 |b|^2)), d = a_qq - a_pp: one square root, one
-          // division and one reciprocal square root in the round's dependent chain
-          const double d = jacobi_re(A[q * ld + q]) - jacobi_re(A[p * ld + p]), b2 = 2.0 * mag;
-          const double r = fabs(d) + sqrt(d * d + b2 * b2);
-          const double tt = r > 0.0 ? copysign(b2 / r, d) : 1.0;
-          c = rsqrt(tt * tt + 1.0);
-          s = tt * c;
-          if constexpr (CPLX) {
-            fr = b.x / mag;
-            fi = b.y / mag;
-          } else if (b < 0.0) {
-            s = -s;
-          }
+      const double2* cs = rot + (round & 1) * half;
+      const int* pq_of = pairs + (round & 1) * half;
+      auto phase = [&](int t) { return CPLX ? cs[2 * half + t] : make_double2(1.0, 0.0); };
+      for (int s = s0, t = t0; s < half;) {
+        const double2 ct = cs[t], ft = phase(t), cr = cs[s], fs = phase(s);
+        const int tp = pq_of[t] & 0xffff, tq = pq_of[t] >> 16, p = pq_of[s] & 0xffff, q = pq_of[s] >> 16;
+        E pp = A[p * ld + tp], pq = A[p * ld + tq], qp = A[q * ld + tp], qq = A[q * ld + tq];
+        jacobi_rotate(pp, qp, cr.x, cr.y, fs.x, fs.y);
+        jacobi_rotate(pq, qq, cr.x, cr.y, fs.x, fs.y);
+        jacobi_rotate(pp, pq, ct.x, ct.y, ft.x, -ft.y);
+        jacobi_rotate(qp, qq, ct.x, ct.y, ft.x, -ft.y);
+        if (s == t && (ct.x != 1.0 || ct.y != 0.0)) {
+          jacobi_set(pq, 0.0);
+          jacobi_set(qp, 0.0);
+          jacobi_drop_imag(pp);
+          jacobi_drop_imag(qq);
         }
-        rot[4 * t] = c;
-        rot[4 * t + 1] = s;
-        rot[4 * t + 2] = fr;
-        rot[4 * t + 3] = fi;
-      }
-      __syncthreads();
-      // blocks (s, t) of A for s < half, then rows 2i, 2i + 1 of V for i = s - half
-      for (int s = s0, t = t0; s < 2 * half;) {
-        const double ct = rot[4 * t], st = rot[4 * t + 1], frt = rot[4 * t + 2], fit = rot[4 * t + 3];
-        int tp, tq;
-        pair_of(t, tp, tq);
-        if (s < half) {
-          const double cs = rot[4 * s], ss = rot[4 * s + 1], frs = rot[4 * s + 2], fis = rot[4 * s + 3];
-          int p, q;
-          pair_of(s, p, q);
-          E pp = A[p * ld + tp], pq = A[p * ld + tq], qp = A[q * ld + tp], qq = A[q * ld + tq];
-          jacobi_rotate(pp, qp, cs, ss, frs, fis);
-          jacobi_rotate(pq, qq, cs, ss, frs, fis);
-          jacobi_rotate(pp, pq, ct, st, frt, -fit);
-          jacobi_rotate(qp, qq, ct, st, frt, -fit);
-          if (s == t && (ct != 1.0 || st != 0.0)) {
-            jacobi_set(pq, 0.0);
-            jacobi_set(qp, 0.0);
-            jacobi_drop_imag(pp);
-            jacobi_drop_imag(qq);
-          }
-          A[p * ld + tp] = pp;
-          A[p * ld + tq] = pq;
-          A[q * ld + tp] = qp;
-          A[q * ld + tq] = qq;
-        } else {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int k = 2 * (s - half) + h;
-            E vp = V[k * ld + tp], vq = V[k * ld + tq];
-            jacobi_rotate(vp, vq, ct, st, frt, -fit);
-            V[k * ld + tp] = vp;
-            V[k * ld + tq] = vq;
-          }
-        }
+        A[p * ld + tp] = pp;
+        A[p * ld + tq] = pq;
+        A[q * ld + tp] = qp;
+        A[q * ld + tq] = qq;
         s += ds;
         t += dt;
         if (t >= half) {
           t -= half;
           ++s;
+        }
+      }
+      __syncthreads();
+      // the next round's angles beside rows 2i, 2i + 1 of V
+      if (va < 0 && round + 2 < np) angles(round + 1);
+      for (int i = i0, t = j0; i < half;) {
+        const double2 ct = cs[t], ft = phase(t);
+        const int tp = pq_of[t] & 0xffff, tq = pq_of[t] >> 16;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          E* row = V + (2 * i + h) * ld;
+          E vp = row[tp], vq = row[tq];
+          jacobi_rotate(vp, vq, ct.x, ct.y, ft.x, -ft.y);
+          row[tp] = vp;
+          row[tq] = vq;
+        }
+        i += di;
+        t += dj;
+        if (t >= half) {
+          t -= half;
+          ++i;
         }
       }
       __syncthreads();
@@ -1381,8 +1401,8 @@ void device_hermitian_eigen(int n, const std::vector<C64>& a, std::vector<double
     }
     QMBED_CUDA(cudaMemcpyAsync(buf, host.data(), nn * w * sizeof(double), cudaMemcpyHostToDevice, stream));
     const int half = (n + 1) / 2;
-    const int items = 2 * half * half, trips = (items + kJacobiMaxThreads - 1) / kJacobiMaxThreads;
-    const int threads = ((items + trips - 1) / trips + 31) / 32 * 32;
+    const int items = half * half, trips = (items + kJacobiBlockItems - 1) / kJacobiBlockItems;
+    const int threads = ((items + trips - 1) / trips + 31) / 32 * 32 + (half + 31) / 32 * 32;
     auto kernel = real ? jacobi_smem_kernel<false> : jacobi_smem_kernel<true>;
     if (smem > 48 * 1024)
       QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
