@@ -108,20 +108,46 @@ __device__ __forceinline__ void dmma_8x8x4(double a, double b, double& c0, doubl
                : "d"(a), "d"(b));
 }
 
+// COUNT consecutive elements in one to two reads (writes) of 8 or 16 bytes.
+template <typename T, int COUNT>
+struct RowPiece {
+  static constexpr int kBytes = COUNT * sizeof(T) >= 16 ? 16 : COUNT * sizeof(T);
+  using Word = std::conditional_t<kBytes == 16, uint4, std::conditional_t<kBytes == 8, uint2, unsigned>>;
+  static constexpr int kWords = COUNT * sizeof(T) / kBytes;
+  union {
+    T v[COUNT];
+    Word words[kWords];
+  };
+  __device__ __forceinline__ void load(const T* p, bool in) {
+#pragma unroll
+    for (int q = 0; q < kWords; ++q) words[q] = in ? __ldg(reinterpret_cast<const Word*>(p) + q) : Word{};
+  }
+  __device__ __forceinline__ void store(T* p) const {
+#pragma unroll
+    for (int q = 0; q < kWords; ++q) reinterpret_cast<Word*>(p)[q] = words[q];
+  }
+};
+
 // The same weighted Gram on the tensor cores. The contraction runs over the
-// rows: every MMA takes 4 consecutive rows of the row-major n x NB blocks, so
-// the 32 lanes' operand loads are the 4 x 8 sub-block of a and of b (one
-// contiguous 256-byte (FP64) or 128-byte (FP32) span per operand). A warp
-// keeps the (NB / 8)^2 output tiles of the NB x NB Gram in registers, strides
-// over groups of 4 rows, and the block reduces its warps in a fixed order.
-template <typename T, int NB>
-__global__ void __launch_bounds__(kThreads) block_gram_mma_kernel(uint64_t n, const T* __restrict__ a,
-                                                                   const T* __restrict__ b,
-                                                                   const uint16_t* __restrict__ weights,
-                                                                   double* __restrict__ partial) {
+// rows: every MMA takes 4 consecutive rows of the row-major n x NB blocks. A
+// lane's columns of the NB / 8 tiles lie next to each other (tile t, column c
+// stands for column c NB / 8 + t), so its operands of a row are one read and
+// the warp's one contiguous span. A warp keeps the output tiles in registers,
+// strides over groups of 4 rows with the next groups' reads in flight, and the
+// block reduces its warps in a fixed order. SAME (a == b): one read of the
+// block, the tiles below the diagonal mirrored.
+//
+// Bound by the FP64 conversions and MMAs next to the panel's read. Measured
+// (B200) at 719 146 rows of 16: FP32 42 -> 17 us (SAME) and 23 us, FP64 43 ->
+// 29 us, against one 4-byte read per operand and tile and no read ahead.
+template <typename T, int NB, bool SAME>
+__global__ void __launch_bounds__(kThreads, 2) block_gram_mma_kernel(uint64_t n, const T* __restrict__ a,
+                                                                      const T* __restrict__ b,
+                                                                      const uint16_t* __restrict__ weights,
+                                                                      double* __restrict__ partial) {
   constexpr int TILES = NB / 8;
   constexpr int kWarps = kThreads / 32;
-  constexpr int kUnroll = 4;  // row groups whose operands are loaded before their MMAs
+  constexpr int kUnroll = 4;  // row groups whose operands are read together
   __shared__ double red[kWarps][NB * NB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, col = lane >> 2;  // operand row within the group, column within a tile
@@ -132,33 +158,48 @@ __global__ void __launch_bounds__(kThreads) block_gram_mma_kernel(uint64_t n, co
     for (int q = 0; q < TILES; ++q) c[p][q][0] = c[p][q][1] = 0.0;
   const uint64_t groups = (n + 3) / 4;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kWarps;
-  for (uint64_t g0 = static_cast<uint64_t>(blockIdx.x) * kWarps + warp; g0 < groups; g0 += stride * kUnroll) {
-    double va[kUnroll][TILES], vb[kUnroll][TILES];
+  RowPiece<T, TILES> xa[kUnroll], xb[SAME ? 1 : kUnroll];
+  unsigned short w[kUnroll];
+  auto read = [&](uint64_t g0) {
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-      const uint64_t g = g0 + u * stride;
-      const uint64_t r = g * 4 + kr;
-      const bool in = g < groups && r < n;
-      const double w = in ? (weights ? static_cast<double>(__ldg(weights + r)) : 1.0) : 0.0;
+      const uint64_t r = (g0 + u * stride) * 4 + kr;
+      const bool in = r < n;
+      xa[u].load(a + r * NB + col * TILES, in);
+      if (!SAME) xb[u].load(b + r * NB + col * TILES, in);
+      w[u] = in && weights ? __ldg(weights + r) : static_cast<unsigned short>(1);
+    }
+  };
+  uint64_t g0 = static_cast<uint64_t>(blockIdx.x) * kWarps + warp;
+  read(g0);
+  while (g0 < groups) {
+    double va[kUnroll][TILES], vb[kUnroll][TILES];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
 #pragma unroll
       for (int t = 0; t < TILES; ++t) {
-        va[u][t] = in ? w * static_cast<double>(__ldg(a + r * NB + t * 8 + col)) : 0.0;
-        vb[u][t] = in ? static_cast<double>(__ldg(b + r * NB + t * 8 + col)) : 0.0;
+        vb[u][t] = static_cast<double>(SAME ? xa[u].v[t] : xb[SAME ? 0 : u].v[t]);
+        va[u][t] = static_cast<double>(w[u]) * (SAME ? vb[u][t] : static_cast<double>(xa[u].v[t]));
       }
-    }
+    g0 += stride * kUnroll;
+    read(g0);
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u)
 #pragma unroll
       for (int p = 0; p < TILES; ++p)
 #pragma unroll
-        for (int q = 0; q < TILES; ++q) dmma_8x8x4(va[u][p], vb[u][q], c[p][q][0], c[p][q][1]);
+        for (int q = SAME ? p : 0; q < TILES; ++q) dmma_8x8x4(va[u][p], vb[u][q], c[p][q][0], c[p][q][1]);
   }
 #pragma unroll
   for (int p = 0; p < TILES; ++p)
 #pragma unroll
-    for (int q = 0; q < TILES; ++q)
+    for (int q = SAME ? p : 0; q < TILES; ++q)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) red[warp][(p * 8 + col) * NB + q * 8 + 2 * kr + h] = c[p][q][h];
+      for (int h = 0; h < 2; ++h) {
+        const int i = col * TILES + p, j = (2 * kr + h) * TILES + q;
+        red[warp][i * NB + j] = c[p][q][h];
+        if (SAME && q != p) red[warp][j * NB + i] = c[p][q][h];
+      }
   __syncthreads();
   for (int t = threadIdx.x; t < NB * NB; t += kThreads) {
     double s = 0.0;
@@ -187,6 +228,7 @@ __global__ void __launch_bounds__(128) reduce_partials_kernel(const double* __re
 // partial[b][q] = sum_r w_r ((w[r][:] C)_q - theta_q out[r][q])^2.
 // Each thread produces 8 outputs of one row (NB / 8 threads per row), which
 // keeps the per-thread state near 100 registers instead of hoisting all of C.
+// The CUDA-core form, selected as the Gram's is; see block_rotate_mma_kernel.
 template <typename T, int NB, bool RESID>
 __global__ void __launch_bounds__(kThreads, 2) block_rotate_kernel(uint64_t n, const T* __restrict__ z,
                                                                     T* __restrict__ out, const T* __restrict__ w,
@@ -276,6 +318,109 @@ __global__ void __launch_bounds__(kThreads, 2) block_rotate_kernel(uint64_t n, c
   }
 }
 
+// The same rotation on the tensor cores: MMAs of 8 rows by 4 of the NB inner
+// columns by 8 outputs, C's operands held in registers for the whole run. Inner
+// step s of lane k stands for column k NB / 4 + s and output 2 k + h of tile t
+// for column k NB / 4 + 2 t + h, so a lane reads and writes one piece of a row
+// and a warp one contiguous span.
+//
+// Bound by the block's read and write next to the FP64 conversions. Measured
+// (B200) at 719 146 rows of 16: FP32 32 -> 16 us, with RESID 56 -> 37, against
+// block_rotate_kernel, which read C from shared memory for every product.
+template <typename T, int NB, bool RESID>
+__global__ void __launch_bounds__(kThreads, 2) block_rotate_mma_kernel(uint64_t n, const T* __restrict__ z,
+                                                                        T* __restrict__ out, const T* __restrict__ w,
+                                                                        const double* __restrict__ coeff,
+                                                                        const double* __restrict__ theta,
+                                                                        const uint16_t* __restrict__ weights,
+                                                                        double* __restrict__ partial) {
+  constexpr int TILES = NB / 8, STEPS = NB / 4;
+  constexpr int kWarps = kThreads / 32;
+  constexpr int kUnroll = RESID ? 2 : 4;
+  __shared__ double red[kWarps][NB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = lane >> 2, part = lane & 3;
+  double c[STEPS][TILES], th[STEPS], res[STEPS];
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+#pragma unroll
+    for (int t = 0; t < TILES; ++t)
+      c[s][t] = coeff[(part * STEPS + s) * NB + (row >> 1) * STEPS + 2 * t + (row & 1)];
+    th[s] = RESID ? theta[part * STEPS + s] : 0.0;
+    res[s] = 0.0;
+  }
+  const uint64_t groups = (n + 7) / 8;
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kWarps;
+  RowPiece<T, STEPS> x[kUnroll], y[RESID ? kUnroll : 1];
+  unsigned short wt[RESID ? kUnroll : 1];
+  auto read = [&](uint64_t g0) {
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const uint64_t r = (g0 + u * stride) * 8 + row;
+      const bool in = r < n;
+      x[u].load(z + r * NB + part * STEPS, in);
+      if constexpr (RESID) {
+        y[u].load(w + r * NB + part * STEPS, in);
+        wt[u] = in && weights ? __ldg(weights + r) : static_cast<unsigned short>(1);
+      }
+    }
+  };
+  uint64_t g0 = static_cast<uint64_t>(blockIdx.x) * kWarps + warp;
+  read(g0);
+  while (g0 < groups) {
+    double a[kUnroll][STEPS], b[RESID ? kUnroll : 1][STEPS], weight[RESID ? kUnroll : 1];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        a[u][s] = static_cast<double>(x[u].v[s]);
+        if constexpr (RESID) b[u][s] = static_cast<double>(y[u].v[s]);
+      }
+      if constexpr (RESID) weight[u] = static_cast<double>(wt[u]);
+    }
+    const uint64_t next = g0 + stride * kUnroll;
+    read(next);
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      double zo[STEPS] = {}, wo[STEPS] = {};
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s)
+#pragma unroll
+        for (int t = 0; t < TILES; ++t) {
+          dmma_8x8x4(a[u][s], c[s][t], zo[2 * t], zo[2 * t + 1]);
+          if constexpr (RESID) dmma_8x8x4(b[u][s], c[s][t], wo[2 * t], wo[2 * t + 1]);
+        }
+      const uint64_t r = (g0 + u * stride) * 8 + row;
+      RowPiece<T, STEPS> to;
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) to.v[s] = static_cast<T>(zo[s]);
+      if (r < n) to.store(out + r * NB + part * STEPS);
+      if constexpr (RESID) {
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) {
+          const double d = wo[s] - th[s] * zo[s];
+          if (r < n) res[s] = fma(weight[u] * d, d, res[s]);
+        }
+      }
+    }
+    g0 = next;
+  }
+  if constexpr (RESID) {
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) {
+      double v = res[s];
+      for (int o = 16; o >= 4; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < 4) red[warp][lane * STEPS + s] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < NB) {
+      double s = 0.0;
+      for (int q = 0; q < kWarps; ++q) s += red[q][threadIdx.x];
+      partial[static_cast<uint64_t>(blockIdx.x) * NB + threadIdx.x] = s;
+    }
+  }
+}
+
 // out[i * n + r] = sqrt(R_r) z[r][i] for i < k (FP64, column-major).
 template <typename T, int NB>
 __global__ void block_export_kernel(uint64_t n, const T* __restrict__ z, int k, const uint16_t* __restrict__ weights,
@@ -341,8 +486,11 @@ class BlockSolver {
       if (scalar)
         block_gram_kernel<T, NB><<<blocks_, kThreads, 0, s>>>(n_, static_cast<const T*>(a), static_cast<const T*>(b),
                                                               op_.weights, partial_.as<double>());
+      else if (a == b)
+        block_gram_mma_kernel<T, NB, true><<<blocks_, kThreads, 0, s>>>(
+            n_, static_cast<const T*>(a), static_cast<const T*>(b), op_.weights, partial_.as<double>());
       else
-        block_gram_mma_kernel<T, NB><<<blocks_, kThreads, 0, s>>>(
+        block_gram_mma_kernel<T, NB, false><<<blocks_, kThreads, 0, s>>>(
             n_, static_cast<const T*>(a), static_cast<const T*>(b), op_.weights, partial_.as<double>());
     });
     QMBED_LAUNCH_CHECK();
@@ -350,7 +498,8 @@ class BlockSolver {
   }
 
   // out = z C (out must not alias z); with `resid` returns the squared
-  // weighted residual norms of (w C) - out diag(theta).
+  // weighted residual norms of (w C) - out diag(theta). On the FP64 tensor
+  // cores as gram() is.
   std::vector<double> rotate(int prec, const void* z, void* out, const void* w, const std::vector<double>& C,
                              const std::vector<double>& theta, bool resid) {
     const cudaStream_t s = ops_.stream();
@@ -359,16 +508,17 @@ class BlockSolver {
     for (size_t q = 0; q < theta.size() && q < static_cast<size_t>(nb_); ++q) host[static_cast<size_t>(nb_) * nb_ + q] = theta[q];
     QMBED_CUDA(cudaMemcpyAsync(coeff_.get(), host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, s));
     const double* c = coeff_.as<double>();
+    const bool scalar = !dense_on_tensor_cores();
     dispatch_block(prec, nb_, [&](auto ttag, auto nbtag) {
       using T = decltype(ttag);
       constexpr int NB = decltype(nbtag)::value;
-      if (resid)
-        block_rotate_kernel<T, NB, true><<<blocks_, kThreads, 0, s>>>(
-            n_, static_cast<const T*>(z), static_cast<T*>(out), static_cast<const T*>(w), c, c + NB * NB,
-            op_.weights, partial_.as<double>());
-      else
-        block_rotate_kernel<T, NB, false><<<blocks_, kThreads, 0, s>>>(
-            n_, static_cast<const T*>(z), static_cast<T*>(out), nullptr, c, nullptr, op_.weights, nullptr);
+      auto launch = [&](auto kernel) {
+        kernel<<<blocks_, kThreads, 0, s>>>(n_, static_cast<const T*>(z), static_cast<T*>(out),
+                                            static_cast<const T*>(w), c, c + NB * NB, op_.weights,
+                                            partial_.as<double>());
+      };
+      if (scalar) launch(resid ? block_rotate_kernel<T, NB, true> : block_rotate_kernel<T, NB, false>);
+      else launch(resid ? block_rotate_mma_kernel<T, NB, true> : block_rotate_mma_kernel<T, NB, false>);
     });
     QMBED_LAUNCH_CHECK();
     if (!resid) return {};

@@ -631,12 +631,13 @@ __global__ void __launch_bounds__(1024) jacobi_kernel(int np, double* __restrict
 // at once; J^H A J splits into the (np/2)^2 independent 2 x 2 blocks (pair s
 // rows, pair t columns), so rows and columns are rotated by one thread per
 // block in one pass. What bounds it is the round's latency chain (shared reads,
-// one division and two square roots per angle, two barriers), not arithmetic:
+// two reciprocal square roots per angle, two barriers), not arithmetic:
 // the projected matrices are 8 to 44 wide. So the warps behind the first one or
 // two rotate the vectors while those compute the next round's angles, and the
 // angles lie as (c, s) pairs, which a warp reads without bank conflicts.
-// Measured (B200): 16 x 16 real 44 us and 44 x 44 real 234 us; 46 and 310 with
-// angles, then blocks and vectors; 210 us and (40 x 40) 2268 us for
+// Measured (B200): 16 x 16 real 39 us and 44 x 44 real 215 us; 44 and 234 with
+// a square root, a division and a reciprocal square root per angle, 46 and 310
+// with angles, then blocks and vectors; 210 us and (40 x 40) 2268 us for
 // jacobi_kernel, which keeps both matrices in global memory as complex numbers;
 // that kernel remains for matrices beyond the shared memory.
 constexpr int kJacobiBlockItems = 512;       // 2 x 2 blocks of a trip
@@ -733,13 +734,19 @@ __global__ void __launch_bounds__(kJacobiMaxThreads)
     const double mag = CPLX ? sqrt(jacobi_sq(b)) : fabs(jacobi_re(b));
     double c = 1.0, s = 0.0, fr = 1.0, fi = 0.0;
     if (mag != 0.0) {
-      // tan = 2 |b| / (d +- sqrt(d^2 + 4 |b|^2)), d = a_qq - a_pp: one square root, one
-      // division and one reciprocal square root in the round's dependent chain
-      const double d = jacobi_re(A[q * ld + q]) - jacobi_re(A[p * ld + p]), b2 = 2.0 * mag;
-      const double r = fabs(d) + sqrt(d * d + b2 * b2);
-      const double tt = r > 0.0 ? copysign(b2 / r, d) : 1.0;
-      c = rsqrt(tt * tt + 1.0);
-      s = tt * c;
+      // cos 2 theta = |d| / sqrt(d^2 + 4 |b|^2), d = a_qq - a_pp: c^2 = (1 + cos 2 theta) / 2
+      // and s = sin 2 theta / (2 c), two reciprocal square roots in the round's dependent chain
+      double d = jacobi_re(A[q * ld + q]) - jacobi_re(A[p * ld + p]), b2 = 2.0 * mag;
+      double x = d * d + b2 * b2;
+      if (!(x > 1e-280 && x < 1e280)) {  // squares out of range: the same ratio from scaled entries
+        const double top = fmax(fabs(d), b2);
+        d /= top;
+        b2 /= top;
+        x = d * d + b2 * b2;
+      }
+      const double u = rsqrt(x), c2 = fma(0.5 * fabs(d), u, 0.5), v = rsqrt(c2);
+      c = c2 * v;
+      s = copysign(0.5 * b2 * u * v, d);
       if constexpr (CPLX) {
         fr = b.x / mag;
         fi = b.y / mag;
