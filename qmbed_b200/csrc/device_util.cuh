@@ -8,6 +8,35 @@ namespace qmbed {
 constexpr int kBinomStride = 129;  // binomial table is [n][k], n,k <= 128
 
 // 16-byte vector access to rows of row-major blocks (addresses 16-byte aligned).
+// First statement of a kernel that launch_dependent() may start while its
+// predecessor in the stream drains: waits until that one has completed and its
+// writes are visible, then lets the next such launch follow. Nothing but the
+// launch's own arguments may be read before it. What the predecessor wrote is
+// read with __ldcg: the non-coherent path asks for data constant over the launch.
+__device__ __forceinline__ void await_previous() {
+#if __CUDA_ARCH__ >= 900
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+#endif
+}
+
+// Launch whose blocks may become resident before the stream's previous kernel
+// has ended (the kernel begins with await_previous()); QMBED_LAUNCH_CHECK follows.
+template <typename... P, typename... A>
+void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  QMBED_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...));
+}
+
 // load16 reads through the read-only path: only for data no thread of the
 // launch writes. load16_rw is the coherent form for rows a launch rewrites.
 __device__ __forceinline__ void load16(const float* p, float (&v)[4]) {

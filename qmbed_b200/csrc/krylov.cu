@@ -59,39 +59,48 @@ __device__ inline double warp_sum(double v) {
 // Overlaps of a tall FP64 panel with one vector, one warp per column: each
 // block stages a slab of `slab` rows of w in shared memory and its warps
 // sweep the columns; every lane keeps eight independent loads in flight.
-// partials[(j * G + block) * 2 + {0,1}] as for multi_dot_kernel.
+// partials[(j * G + block) * 2 + {0,1}] as for multi_dot_kernel. Bound by the
+// panel's read (kept_columns: the last `keep` columns stay in the L2): 44.7 us
+// on average for 1 to 100 columns of 718,146 rows, 42 with the kept columns.
 constexpr int kMaxSlab = 2048;
 template <bool CPLX>
 __global__ void __launch_bounds__(kThreads) panel_dot_kernel(const double* __restrict__ A, uint64_t ld, int m,
                                                              const double* __restrict__ w, uint64_t n, int slab,
-                                                             double* __restrict__ partials) {
+                                                             int keep, double* __restrict__ partials) {
   constexpr int W = CPLX ? 2 : 1;
   extern __shared__ __align__(16) double ws[];
   const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * slab;
   const int rows = static_cast<int>(min(static_cast<uint64_t>(slab), n - r0));
-  for (int t = threadIdx.x; t < rows * W; t += blockDim.x) ws[t] = w[r0 * W + t];
+  await_previous();
+  for (int t = threadIdx.x; t < rows * W; t += blockDim.x) ws[t] = __ldcg(w + r0 * W + t);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const uint64_t G = gridDim.x;
   for (int j = threadIdx.x >> 5; j < m; j += kThreads / 32) {
     const double* q = A + static_cast<uint64_t>(j) * ld * W + r0 * W;
     double sr = 0.0, si = 0.0;
-    for (int r = lane; r < rows; r += 32 * 8) {
+    auto sweep = [&](auto stream) {
+      constexpr bool STREAM = decltype(stream)::value;
+      for (int r = lane; r < rows; r += 32 * 8) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = r + 32 * u;
-        if (k < rows) {
-          if (CPLX) {
-            const double2 x = reinterpret_cast<const double2*>(q)[k];
-            const double2 y = reinterpret_cast<const double2*>(ws)[k];
-            sr += x.x * y.x + x.y * y.y;
-            si += x.x * y.y - x.y * y.x;
-          } else {
-            sr += q[k] * ws[k];
+        for (int u = 0; u < 8; ++u) {
+          const int k = r + 32 * u;
+          if (k < rows) {
+            if (CPLX) {
+              const double2* at = reinterpret_cast<const double2*>(q) + k;
+              const double2 x = STREAM ? __ldcs(at) : __ldg(at);
+              const double2 y = reinterpret_cast<const double2*>(ws)[k];
+              sr += x.x * y.x + x.y * y.y;
+              si += x.x * y.y - x.y * y.x;
+            } else {
+              sr += (STREAM ? __ldcs(q + k) : __ldg(q + k)) * ws[k];
+            }
           }
         }
       }
-    }
+    };
+    if (j < m - keep) sweep(std::true_type{});
+    else sweep(std::false_type{});
     sr = warp_sum(sr);
     if (CPLX) si = warp_sum(si);
     if (lane == 0) {
@@ -168,10 +177,11 @@ constexpr int kFinishThreads = 128;
 __global__ void __launch_bounds__(kFinishThreads) finish_kernel(const double* __restrict__ partials, int G, int count,
                                                                 double* __restrict__ out) {
   const int t = blockIdx.x;
+  await_previous();
   if (t >= count) return;
   const int j = t / 2, c = t & 1;
   double total = 0.0;
-  for (int b = threadIdx.x; b < G; b += kFinishThreads) total += partials[(static_cast<uint64_t>(j) * G + b) * 2 + c];
+  for (int b = threadIdx.x; b < G; b += kFinishThreads) total += __ldcg(partials + (static_cast<uint64_t>(j) * G + b) * 2 + c);
   __shared__ double tree[kFinishThreads];
   tree[threadIdx.x] = total;
   __syncthreads();
@@ -863,6 +873,17 @@ int stream_grid(uint64_t n, int sms) {
   return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(blocks, static_cast<uint64_t>(8) * sms)));
 }
 
+// Columns that stay in the L2 between the sweeps of a panel: the overlaps go up
+// the columns, the subtraction down, so each sweep begins with the columns that
+// the other one ended with. Those are read as usual, the others evict-first (a
+// sweep over a panel beyond the L2 drives out the columns it is about to need
+// otherwise). Two Lanczos runs of 100 steps at 718,146 rows (28 sites): 26.5 ms
+// without, 25.4 at 30 MB, 25.3 at 40 to 50, 25.5 at 70, 26.6 with none kept.
+int kept_columns(uint64_t n, bool cplx) {
+  constexpr uint64_t kKeptPanelBytes = 48ull << 20;
+  return static_cast<int>(std::min<uint64_t>(kKeptPanelBytes / (n * (cplx ? 16 : 8)), 1u << 20));
+}
+
 constexpr int kOrthoThreads = 256;
 constexpr int kOrthoChunk = 8;
 
@@ -887,86 +908,109 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // |src - sum_k h_k q_k|^2. Elements are complex values
 // (kComplex), pairs of real rows loaded as one 16-byte word (kRealPair, n
 // even), or single real rows (kReal).
+//
+// Bound by the panel's read. The columns are taken from the last down, `keep`
+// of them from what the overlaps' sweep left in the L2 (kept_columns), and a
+// thread takes ROWS elements along, so that the grid sweeps the columns once
+// instead of once per grid stride: 718,146 rows by 1 to 100 columns (28 sites)
+// 48.9 -> 46.6 us on average, 6.2 TB/s, and 44 with the kept columns.
 enum { kReal = 0, kRealPair = 1, kComplex = 2 };
-template <int MODE>
+template <int MODE, int ROWS>
 __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const double* __restrict__ Q, uint64_t n, int m,
                                                                       const double* __restrict__ h, double beta_value,
                                                                       const double* __restrict__ beta_device,
-                                                                      int before_mode, const double* src,
+                                                                      int before_mode, int keep, const double* src,
                                                                       double* w, double* __restrict__ partials) {
   extern __shared__ double hs[];
   __shared__ double red[kOrthoThreads / 32];
-  for (int t = threadIdx.x; t < 2 * m; t += blockDim.x) hs[t] = h[t];
+  await_previous();
+  for (int t = threadIdx.x; t < 2 * m; t += blockDim.x) hs[t] = __ldcg(h + t);
   __syncthreads();
   const double alpha = hs[2 * (m - 1)];
-  const double beta = beta_device ? *beta_device : beta_value;
+  const double beta = beta_device ? __ldcg(beta_device) : beta_value;
   // element count and the stride between columns, in elements
   const uint64_t elems = MODE == kRealPair ? n / 2 : n;
   const uint64_t col = MODE == kReal ? n : n / (MODE == kRealPair ? 2 : 1);
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  // columns loaded ahead per element: eight 8-byte or four 16-byte words
-  constexpr int CH = MODE == kReal ? kOrthoChunk : kOrthoChunk / 2;
+  // columns loaded ahead per element: eight 8-byte or four 16-byte words in all
+  constexpr int CH = (MODE == kReal ? kOrthoChunk : kOrthoChunk / 2) / (ROWS > 1 ? 2 : 1);
   double before = 0.0, after = 0.0;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < elems; i += stride) {
+  for (uint64_t i0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < elems; i0 += ROWS * stride) {
     // (a, b): real and imaginary parts, or the two rows of a pair
-    double wa, wb = 0.0;
-    if (MODE == kReal) {
-      wa = src[i];
-    } else {
-      const double2 v = reinterpret_cast<const double2*>(src)[i];
-      wa = v.x;
-      wb = v.y;
-    }
-    double sa = 0.0, sb = 0.0, la = 0.0, lb = 0.0, pa = 0.0, pb = 0.0;
-    // from the last columns down: the overlaps' sweep left those in the L2
-    for (int j0 = (m - 1) / CH * CH; j0 >= 0; j0 -= CH) {
-      double xa[CH], xb[CH];
+    double sa[ROWS], sb[ROWS], ta[ROWS], tb[ROWS];  // the pass's sum, the three-term one
 #pragma unroll
-      for (int jj = 0; jj < CH; ++jj) {
-        xa[jj] = xb[jj] = 0.0;
-        if (j0 + jj < m) {
-          if (MODE == kReal) {
-            xa[jj] = Q[static_cast<uint64_t>(j0 + jj) * col + i];
-          } else {
-            const double2 v = reinterpret_cast<const double2*>(Q)[static_cast<uint64_t>(j0 + jj) * col + i];
-            xa[jj] = v.x;
-            xb[jj] = v.y;
+    for (int u = 0; u < ROWS; ++u) sa[u] = sb[u] = ta[u] = tb[u] = 0.0;
+    for (int j0 = (m - 1) / CH * CH; j0 >= 0; j0 -= CH) {
+      double xa[CH][ROWS], xb[CH][ROWS];
+      auto read = [&](auto stream) {
+        constexpr bool STREAM = decltype(stream)::value;
+#pragma unroll
+        for (int jj = 0; jj < CH; ++jj)
+#pragma unroll
+          for (int u = 0; u < ROWS; ++u) {
+            const uint64_t i = i0 + u * stride;
+            xa[jj][u] = xb[jj][u] = 0.0;
+            if (j0 + jj < m && (ROWS == 1 || i < elems)) {
+              if (MODE == kReal) {
+                const double* q = Q + static_cast<uint64_t>(j0 + jj) * col + i;
+                xa[jj][u] = STREAM ? __ldcs(q) : __ldg(q);
+              } else {
+                const double2* q = reinterpret_cast<const double2*>(Q) + static_cast<uint64_t>(j0 + jj) * col + i;
+                const double2 v = STREAM ? __ldcs(q) : __ldg(q);
+                xa[jj][u] = v.x;
+                xb[jj][u] = v.y;
+              }
+            }
           }
-        }
-      }
+      };
+      if (j0 >= keep) read(std::true_type{});
+      else read(std::false_type{});
 #pragma unroll
       for (int jj = 0; jj < CH; ++jj) {
         const int k = j0 + jj;
         if (k < m) {
           const double hr = hs[2 * k], hi = hs[2 * k + 1];
-          if (MODE == kComplex) {
-            sa += hr * xa[jj] - hi * xb[jj];
-            sb += hr * xb[jj] + hi * xa[jj];
-          } else {  // real basis: the overlaps are real
-            sa += hr * xa[jj];
-            sb += hr * xb[jj];
-          }
-          if (k == m - 1) {
-            la = xa[jj];
-            lb = xb[jj];
-          }
-          if (k == m - 2) {
-            pa = xa[jj];
-            pb = xb[jj];
+#pragma unroll
+          for (int u = 0; u < ROWS; ++u) {
+            if (MODE == kComplex) {
+              sa[u] += hr * xa[jj][u] - hi * xb[jj][u];
+              sb[u] += hr * xb[jj][u] + hi * xa[jj][u];
+            } else {  // real basis: the overlaps are real
+              sa[u] += hr * xa[jj][u];
+              sb[u] += hr * xb[jj][u];
+            }
+            if (k >= m - 2) {
+              const double t = k == m - 1 ? alpha : beta;
+              ta[u] += t * xa[jj][u];
+              tb[u] += t * xb[jj][u];
+            }
           }
         }
       }
     }
-    if (before_mode == 1) {
-      const double ba = wa - alpha * la - beta * pa, bb = wb - alpha * lb - beta * pb;
-      before += ba * ba + bb * bb;
-    } else if (before_mode == 2) {
-      before += wa * wa + wb * wb;
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const uint64_t i = i0 + u * stride;
+      if (ROWS > 1 && i >= elems) break;
+      double wa, wb = 0.0;
+      if (MODE == kReal) {
+        wa = src[i];
+      } else {
+        const double2 v = reinterpret_cast<const double2*>(src)[i];
+        wa = v.x;
+        wb = v.y;
+      }
+      if (before_mode == 1) {
+        const double ba = wa - ta[u], bb = wb - tb[u];
+        before += ba * ba + bb * bb;
+      } else if (before_mode == 2) {
+        before += wa * wa + wb * wb;
+      }
+      const double ra = wa - sa[u], rb = wb - sb[u];
+      if (MODE == kReal) w[i] = ra;
+      else reinterpret_cast<double2*>(w)[i] = make_double2(ra, rb);
+      after += ra * ra + rb * rb;
     }
-    const double ra = wa - sa, rb = wb - sb;
-    if (MODE == kReal) w[i] = ra;
-    else reinterpret_cast<double2*>(w)[i] = make_double2(ra, rb);
-    after += ra * ra + rb * rb;
   }
   before = block_sum(before, red);
   after = block_sum(after, red);
@@ -974,6 +1018,38 @@ __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const d
     partials[2 * blockIdx.x] = before;
     partials[2 * blockIdx.x + 1] = after;
   }
+}
+
+// Launches orthogonalize_kernel and returns its grid (partials: two per block).
+// Elements a thread takes along: as many as one resident grid (four blocks an
+// SM) needs for one sweep, three at most.
+int launch_orthogonalize(const double* A, uint64_t n, int m, const double* h, double beta, const double* beta_device,
+                         int before_mode, const double* src, double* w, double* partials, bool cplx, int sms,
+                         cudaStream_t stream) {
+  // pairs of real rows move as 16-byte words when every column starts 16-byte aligned
+  const int mode = cplx ? kComplex : (n % 2 == 0 ? kRealPair : kReal);
+  const uint64_t elems = mode == kRealPair ? n / 2 : n, resident = 4ull * sms * kOrthoThreads;
+  const int rows = static_cast<int>(std::min<uint64_t>(3, (elems + resident - 1) / resident));
+  const uint64_t per_block = static_cast<uint64_t>(rows) * kOrthoThreads;
+  const int G = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((elems + per_block - 1) / per_block, 4ull * sms)));
+  const size_t smem = static_cast<size_t>(m) * 16;
+  auto launch = [&](auto kernel) {
+    if (smem > 48 * 1024)
+      QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    launch_dependent(kernel, G, kOrthoThreads, smem, stream, A, n, m, h, beta, beta_device, before_mode,
+                     kept_columns(n, cplx), src, w, partials);
+  };
+  auto by_rows = [&](auto mode_tag) {
+    constexpr int MODE = decltype(mode_tag)::value;
+    if (rows == 1) launch(orthogonalize_kernel<MODE, 1>);
+    else if (rows == 2) launch(orthogonalize_kernel<MODE, 2>);
+    else launch(orthogonalize_kernel<MODE, 3>);
+  };
+  if (mode == kComplex) by_rows(std::integral_constant<int, kComplex>{});
+  else if (mode == kRealPair) by_rows(std::integral_constant<int, kRealPair>{});
+  else by_rows(std::integral_constant<int, kReal>{});
+  QMBED_LAUNCH_CHECK();
+  return G;
 }
 
 // out[0..1] = sums of the two partial columns over G blocks (fixed order);
@@ -1005,17 +1081,26 @@ __global__ void __launch_bounds__(128) orthogonalize_finish_kernel(const double*
   }
 }
 
-// The record of a queued step: norms before and after, the DGKS verdict and the last overlap.
-__global__ void __launch_bounds__(128) lanczos_record_kernel(const double* __restrict__ partials, int G, int m,
-                                                             const double* __restrict__ h, double* __restrict__ record) {
+// End of a queued step: every block sums the norms' partials in the same order,
+// the first writes the record (norms before and after, the DGKS verdict and the
+// last overlap), all scale the vector into the next column. One launch; a
+// record kernel of its own took 3.2 us and a gap in front of the scaling.
+__global__ void __launch_bounds__(kThreads) scale_and_record_kernel(const double* __restrict__ partials, int G, int m,
+                                                                    const double* __restrict__ h,
+                                                                    double* __restrict__ record,
+                                                                    const double* __restrict__ src,
+                                                                    double* __restrict__ dst, uint64_t count) {
   __shared__ double tree[2][128];
-  double b = 0.0, a = 0.0;
-  for (int k = threadIdx.x; k < G; k += 128) {
-    b += partials[2 * k];
-    a += partials[2 * k + 1];
+  await_previous();
+  if (threadIdx.x < 128) {
+    double b = 0.0, a = 0.0;
+    for (int k = threadIdx.x; k < G; k += 128) {
+      b += __ldcg(partials + 2 * k);
+      a += __ldcg(partials + 2 * k + 1);
+    }
+    tree[0][threadIdx.x] = b;
+    tree[1][threadIdx.x] = a;
   }
-  tree[0][threadIdx.x] = b;
-  tree[1][threadIdx.x] = a;
   __syncthreads();
   for (int width = 64; width > 0; width >>= 1) {
     if (threadIdx.x < width) {
@@ -1024,26 +1109,20 @@ __global__ void __launch_bounds__(128) lanczos_record_kernel(const double* __res
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    const double before = sqrt(fmax(tree[0][0], 0.0)), after = sqrt(fmax(tree[1][0], 0.0));
+  const double before = sqrt(fmax(tree[0][0], 0.0)), after = sqrt(fmax(tree[1][0], 0.0));
+  const bool ok = isfinite(after) && after > 1.0e-14;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     record[0] = before;
     record[1] = after;
     record[2] = before > 2.220446049250313e-16 && after <= 0.70710678118654752440 * before ? 1.0 : 0.0;
-    record[3] = isfinite(after) && after > 1.0e-14 ? 1.0 : 0.0;
-    record[FusedOrtho::kRecordHead + 2 * (m - 1)] = h[0];
-    record[FusedOrtho::kRecordHead + 2 * (m - 1) + 1] = h[1];
+    record[3] = ok ? 1.0 : 0.0;
+    record[FusedOrtho::kRecordHead + 2 * (m - 1)] = __ldcg(h);
+    record[FusedOrtho::kRecordHead + 2 * (m - 1) + 1] = __ldcg(h + 1);
   }
-}
-
-// dst = src / the record's norm
-__global__ void __launch_bounds__(kThreads) scale_by_record_kernel(const double* __restrict__ src,
-                                                                   double* __restrict__ dst, uint64_t count,
-                                                                   const double* __restrict__ record) {
-  if (record[3] == 0.0) return;
-  const double divisor = record[1];
+  if (!ok) return;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride)
-    dst[i] = src[i] / divisor;
+    dst[i] = __ldcg(src + i) / after;
 }
 
 }  // namespace
@@ -1205,13 +1284,11 @@ void BlockOps::dots_device(const void* A, uint64_t ld, int m, const void* w, uin
     ensure_partials(static_cast<size_t>(m) * G * 2 + 2 * static_cast<size_t>(m) + 64);
     const size_t smem = static_cast<size_t>(slab) * (cplx ? 16 : 8);
     if (cplx)
-      panel_dot_kernel<true><<<G, kThreads, smem, stream_>>>(static_cast<const double*>(A), ld, m,
-                                                             static_cast<const double*>(w), n, slab,
-                                                             partials_.as<double>());
+      launch_dependent(panel_dot_kernel<true>, G, kThreads, smem, stream_, static_cast<const double*>(A), ld, m,
+                       static_cast<const double*>(w), n, slab, kept_columns(n, cplx), partials_.as<double>());
     else
-      panel_dot_kernel<false><<<G, kThreads, smem, stream_>>>(static_cast<const double*>(A), ld, m,
-                                                              static_cast<const double*>(w), n, slab,
-                                                              partials_.as<double>());
+      launch_dependent(panel_dot_kernel<false>, G, kThreads, smem, stream_, static_cast<const double*>(A), ld, m,
+                       static_cast<const double*>(w), n, slab, kept_columns(n, cplx), partials_.as<double>());
   } else {
     G = reduction_grid(n, sms_);
     ensure_partials(static_cast<size_t>(m) * G * 2 + 2 * static_cast<size_t>(m) + 64);
@@ -1221,7 +1298,7 @@ void BlockOps::dots_device(const void* A, uint64_t ld, int m, const void* w, uin
                                                                         partials_.as<double>(), 0)));
   }
   QMBED_LAUNCH_CHECK();
-  finish_kernel<<<2 * m, kFinishThreads, 0, stream_>>>(partials_.as<double>(), G, 2 * m, out);
+  launch_dependent(finish_kernel, 2 * m, kFinishThreads, 0, stream_, partials_.as<double>(), G, 2 * m, out);
   QMBED_LAUNCH_CHECK();
 }
 
@@ -1479,19 +1556,8 @@ void BlockOps::gram_schmidt_pass(const double* A, uint64_t n, int m, double beta
   ensure_coeffs(static_cast<size_t>(m) * 16);
   double* h = coeffs_.as<double>();
   dots_device(A, n, m, w, n, 64, cplx, h);
-  const int G = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kOrthoThreads - 1) / kOrthoThreads,
-                                                                          4ull * sms_)));
-  ensure_partials(2 * static_cast<size_t>(G) + 64);
-  // pairs of real rows move as 16-byte words when every column starts 16-byte aligned
-  const int mode = cplx ? kComplex : (n % 2 == 0 ? kRealPair : kReal);
-  auto kernel = mode == kComplex ? orthogonalize_kernel<kComplex>
-                                 : (mode == kRealPair ? orthogonalize_kernel<kRealPair> : orthogonalize_kernel<kReal>);
-  const size_t smem = static_cast<size_t>(m) * 16;
-  if (smem > 48 * 1024)
-    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, h, beta, nullptr, three_term ? 1 : 0, w, w,
-                                               partials_.as<double>());
-  QMBED_LAUNCH_CHECK();
+  ensure_partials(8 * static_cast<size_t>(sms_) + 64);
+  const int G = launch_orthogonalize(A, n, m, h, beta, nullptr, three_term ? 1 : 0, w, w, partials_.as<double>(), cplx, sms_, stream_);
   orthogonalize_finish_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, h + 2 * (m - 1),
                                                       results_.as<double>());
   QMBED_LAUNCH_CHECK();
@@ -1512,22 +1578,11 @@ void BlockOps::lanczos_step(const double* A, uint64_t n, int m, double* w, doubl
   ensure_coeffs(static_cast<size_t>(m) * 16);
   double* h = coeffs_.as<double>();
   dots_device(A, n, m, w, n, 64, cplx, h);
-  const int G = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kOrthoThreads - 1) / kOrthoThreads,
-                                                                          4ull * sms_)));
-  ensure_partials(2 * static_cast<size_t>(G) + 64);
-  const int mode = cplx ? kComplex : (n % 2 == 0 ? kRealPair : kReal);
-  auto kernel = mode == kComplex ? orthogonalize_kernel<kComplex>
-                                 : (mode == kRealPair ? orthogonalize_kernel<kRealPair> : orthogonalize_kernel<kReal>);
-  const size_t smem = static_cast<size_t>(m) * 16;
-  if (smem > 48 * 1024)
-    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, h, 0.0, beta, 1, w, w, partials_.as<double>());
-  QMBED_LAUNCH_CHECK();
-  lanczos_record_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, m, h + 2 * (m - 1), record);
-  QMBED_LAUNCH_CHECK();
-  if (!slot) return;
-  const uint64_t count = n * (cplx ? 2 : 1);
-  scale_by_record_kernel<<<stream_grid(count, sms_), kThreads, 0, stream_>>>(w, slot, count, record);
+  ensure_partials(8 * static_cast<size_t>(sms_) + 64);
+  const int G = launch_orthogonalize(A, n, m, h, 0.0, beta, 1, w, w, partials_.as<double>(), cplx, sms_, stream_);
+  const uint64_t count = slot ? n * (cplx ? 2 : 1) : 0;
+  launch_dependent(scale_and_record_kernel, slot ? stream_grid(count, sms_) : 1, kThreads, 0, stream_,
+                   partials_.as<double>(), G, m, h + 2 * (m - 1), record, w, slot, count);
   QMBED_LAUNCH_CHECK();
 }
 
@@ -1537,17 +1592,8 @@ void BlockOps::project_out(const double* A, uint64_t n, int m, const double* src
   ensure_coeffs(static_cast<size_t>(m) * 16);
   double* hd = coeffs_.as<double>();
   dots_device(A, n, m, src, n, 64, cplx, hd);
-  const int G = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kOrthoThreads - 1) / kOrthoThreads,
-                                                                          4ull * sms_)));
-  ensure_partials(2 * static_cast<size_t>(G) + 2 * static_cast<size_t>(m) + 64);
-  const int mode = cplx ? kComplex : (n % 2 == 0 ? kRealPair : kReal);
-  auto kernel = mode == kComplex ? orthogonalize_kernel<kComplex>
-                                 : (mode == kRealPair ? orthogonalize_kernel<kRealPair> : orthogonalize_kernel<kReal>);
-  const size_t smem = static_cast<size_t>(m) * 16;
-  if (smem > 48 * 1024)
-    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<G, kOrthoThreads, smem, stream_>>>(A, n, m, hd, 0.0, nullptr, 2, src, w, partials_.as<double>());
-  QMBED_LAUNCH_CHECK();
+  ensure_partials(8 * static_cast<size_t>(sms_) + 2 * static_cast<size_t>(m) + 64);
+  const int G = launch_orthogonalize(A, n, m, hd, 0.0, nullptr, 2, src, w, partials_.as<double>(), cplx, sms_, stream_);
   orthogonalize_finish_kernel<<<1, 128, 0, stream_>>>(partials_.as<double>(), G, hd, results_.as<double>());
   QMBED_LAUNCH_CHECK();
   QMBED_CUDA(cudaMemcpyAsync(host_results_, results_.get(), 2 * sizeof(double), cudaMemcpyDeviceToHost, stream_));
