@@ -519,6 +519,7 @@ __global__ void __launch_bounds__((1 << VB) / kWordsPerThread) flip_box_kernel(c
   __shared__ __align__(8) uint64_t full;
   __shared__ double dword[1 << (VB - kBoxLaneBits)];
   const uint64_t id = blockIdx.x;
+  await_previous();
   if (threadIdx.x == 0) {
     mbar_init(&full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -588,6 +589,7 @@ __global__ void __launch_bounds__(kPassThreads, 3) flip_group_kernel(const __gri
   const int run_bits = 2 + a.bb;
   const int batch_shift = a.b0 - VBITS - run_bits;
   const uint64_t blk = blockIdx.x & ((1ull << batch_shift) - 1), above = static_cast<uint64_t>(blockIdx.x) >> batch_shift;
+  await_previous();
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; ++j) mbar_init(&full[j], 1);
@@ -836,9 +838,9 @@ void launch_box_plan(BoxArgs<T> base, const BoxPlan& plan, double alpha, const s
   for (int i = 0; i < VBITS; ++i) base.cinside[i] = host_coef<T>(alpha * xc[i]);
   for (int i = 0; i < plan.extra; ++i) base.cextra[i] = host_coef<T>(alpha * xc[VBITS + plan.vb + i]);
   const unsigned boxes = 1u << (sites - VBITS - plan.vb);
-  if (plan.vb == 8) flip_box_kernel<T, C, 8, false><<<boxes, 32, 0, stream>>>(base);
-  else if (plan.far_first) flip_box_kernel<T, C, 10, sizeof(T) == 4><<<boxes, 128, 0, stream>>>(base);
-  else flip_box_kernel<T, C, 10, false><<<boxes, 128, 0, stream>>>(base);
+  if (plan.vb == 8) launch_dependent(flip_box_kernel<T, C, 8, false>, boxes, 32, 0, stream, base);
+  else if (plan.far_first) launch_dependent(flip_box_kernel<T, C, 10, sizeof(T) == 4>, boxes, 128, 0, stream, base);
+  else launch_dependent(flip_box_kernel<T, C, 10, false>, boxes, 128, 0, stream, base);
   QMBED_LAUNCH_CHECK();
   if (plan.groups.empty()) return;
   constexpr int kSmem = 16 << kBoxMaxWords;
@@ -857,7 +859,7 @@ void launch_box_plan(BoxArgs<T> base, const BoxPlan& plan, double alpha, const s
     for (int i = g.lo; i < kBoxMaxWords; ++i) g.cbit[i] = host_coef<T>(alpha * xc[b0 + i - g.lo]);
     const CUtensorMap map =
         group_map(base.x, sites, static_cast<int>(sizeof(T)) * (C ? 2 : 1), VBITS + 2, g.b0, g.G, g.bb);
-    group<<<1u << (sites - VBITS - kBoxMaxWords), kPassThreads, kSmem, stream>>>(map, g);
+    launch_dependent(group, 1u << (sites - VBITS - kBoxMaxWords), kPassThreads, kSmem, stream, map, g);
     QMBED_LAUNCH_CHECK();
     b0 += G;
   }

@@ -1328,6 +1328,7 @@ __global__ void __launch_bounds__(kExchangeThreads) exchange_row_kernel(const __
   }
   for (int i = threadIdx.x; i < a.rank_chunks * kRankChunkValues * a.rank_stride; i += blockDim.x)
     s_rank[i] = static_cast<uint32_t>(__ldg(a.rank_tab + i));
+  await_previous();  // what is read above was complete when the basis and its table were built
   __syncthreads();
 
   const int L = a.sites;
@@ -1979,7 +1980,7 @@ bool launch_exchange(const SpinBasis& basis, const DeviceFlipProgram& prog, cons
     }
     const uint64_t needed = (a.rows + kExchangeThreads - 1) / kExchangeThreads;
     const uint64_t cap = static_cast<uint64_t>(cached_sms) * std::max(cached_per_sm, 1);
-    kernel<<<static_cast<unsigned>(std::min(needed, cap)), kExchangeThreads, smem, l.stream>>>(a);
+    launch_dependent(kernel, static_cast<unsigned>(std::min(needed, cap)), kExchangeThreads, smem, l.stream, a);
     QMBED_LAUNCH_CHECK();
   };
   auto by_holes = [&](auto t, auto st, auto c1, auto c2, auto c3) {

@@ -430,14 +430,8 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
   for (int u = 0; u < KB; ++u) e[u] = from + u < to ? load_entry(row + (from + u) * 32) : kNoEntry;
   T xr = 0, xi = 0, dr = 0, di = 0;
   uint32_t orbit = 0;
-  if (valid && (SPLIT == 1 || warp == 0)) {
-    if (VC) {
-      const P v = load_complex<T, VEC2>(x, r);
-      xr = v.x;
-      xi = v.y;
-    } else {
-      xr = __ldg(x + r);
-    }
+  const bool own = valid && (SPLIT == 1 || warp == 0);
+  if (own) {
     if (VALC) {
       dr = __ldcs(diag + 2 * r);
       di = __ldcs(diag + 2 * r + 1);
@@ -453,6 +447,16 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
       table[i].y = static_cast<T>(v.y);
     } else {
       table[i] = static_cast<T>(v.x);
+    }
+  }
+  await_previous();
+  if (own) {
+    if (VC) {
+      const P v = load_complex<T, VEC2>(x, r);
+      xr = v.x;
+      xi = v.y;
+    } else {
+      xr = __ldg(x + r);
     }
   }
   __syncthreads();
@@ -558,6 +562,7 @@ __global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32
 #pragma unroll
   for (int u = 0; u < KB; ++u) e[u] = u < width ? __ldg(row + u * 32) : kNoEntry;
   for (int i = threadIdx.x; i < codes; i += blockDim.x) table[i] = static_cast<T>(values[i].x);
+  await_previous();
   __syncthreads();
   if (r >= n) return;
   T acc[VEC];
@@ -846,9 +851,9 @@ void launch_spmv(const TileRows& rows, const SpinBasis& basis, const double* sqr
   const double2* values = rows.values.as<double2>() + rows.codes;
   const uint16_t* orbits = basis.symmetric() ? basis.orbits() : nullptr;
   auto launch = [&](auto kernel, uint64_t blocks) {
-    kernel<<<static_cast<unsigned>(blocks), kSpmvThreads, smem, stream>>>(
-        rows.n, rows.tile_ptr.as<uint32_t>(), rows.entries.as<uint32_t>(), rows.col_bits, values, rows.codes, diag,
-        orbits, sqrt_table, static_cast<const T*>(x), static_cast<T*>(y));
+    launch_dependent(kernel, static_cast<unsigned>(blocks), kSpmvThreads, smem, stream, rows.n,
+                     rows.tile_ptr.as<uint32_t>(), rows.entries.as<uint32_t>(), rows.col_bits, values, rows.codes, diag,
+                     orbits, sqrt_table, static_cast<const T*>(x), static_cast<T*>(y));
   };
   constexpr int kWarps = kSpmvThreads / 32;
   const uint64_t blocks = (tiles + kWarps - 1) / kWarps;
@@ -898,11 +903,11 @@ void tile_spmm(const TileRows& rows, int shape, int precision, int nb, const voi
     const unsigned grid = static_cast<unsigned>((warps + threads / 32 - 1) / (threads / 32));
     const T* diag = precision == 64 ? reinterpret_cast<const T*>(rows.diag64.get())
                                     : reinterpret_cast<const T*>(rows.diag32.get());
-    tile_spmm_kernel<T, NB, HP, decltype(kbtag)::value>
-        <<<grid, threads, static_cast<size_t>(rows.codes) * sizeof(T), stream>>>(
-            rows.n, rows.tile_ptr.as<uint32_t>(), rows.entries.as<uint32_t>(), rows.col_bits,
-            rows.values.as<double2>(), rows.codes, diag, static_cast<const T*>(z), static_cast<const T*>(p),
-            static_cast<T*>(out), static_cast<T>(alpha), static_cast<T>(beta), static_cast<T>(gamma));
+    launch_dependent(tile_spmm_kernel<T, NB, HP, decltype(kbtag)::value>, grid, threads,
+                     static_cast<size_t>(rows.codes) * sizeof(T), stream, rows.n, rows.tile_ptr.as<uint32_t>(),
+                     rows.entries.as<uint32_t>(), rows.col_bits, rows.values.as<double2>(), rows.codes, diag,
+                     static_cast<const T*>(z), static_cast<const T*>(p), static_cast<T*>(out),
+                     static_cast<T>(alpha), static_cast<T>(beta), static_cast<T>(gamma));
   };
   auto by_kb = [&](auto ttag, auto nbtag, auto ptag) {
     if (kBatchOf[shape] == 8) launch(ttag, nbtag, ptag, std::integral_constant<int, 8>{});
