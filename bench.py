@@ -779,11 +779,11 @@ def main():
         del zb, pb
 
     if block:
-        kernel, achieved_top = "spmm_packed_kernel (FP32 block action, 8 vectors)", block["gbs"]
-        traffic_file = ROOT / "profiles" / f"spmm_packed_L{sites}_traffic.json"
+        kernel, achieved_top = "tile_spmm_kernel (FP32 block action, 8 vectors)", block["gbs"]
+        traffic_file = ROOT / "profiles" / f"tile_spmm_L{sites}_traffic.json"
     else:
-        kernel, achieved_top = "spmv_packed_kernel (FP32 H.v)", achieved
-        traffic_file = ROOT / "profiles" / f"spmv_packed_L{sites}_traffic.json"
+        kernel, achieved_top = "tile_spmv_kernel (FP32 H.v)", achieved
+        traffic_file = ROOT / "profiles" / f"tile_spmv_L{sites}_traffic.json"
     traffic = None
     if traffic_file.exists():
         traffic = json.loads(traffic_file.read_text()).get("dram_bytes_per_launch")

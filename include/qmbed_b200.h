@@ -188,7 +188,7 @@ QMBED_API int qmbed_gpu_operator_operand_bytes(qmbed_operator op, int precision,
  * does not fit), QMBED_LOOKUP_SEARCH, QMBED_LOOKUP_LEGACY (one thread per row
  * over every product, the form used for u128 states and products that repeat
  * a site), QMBED_LOOKUP_TABLE_GENERIC (the table with the general tile kernel
- * even where the nearest-neighbour hop kernel applies). */
+ * even where the kernels for neighbour chains apply). */
 #define QMBED_LOOKUP_AUTO 0
 #define QMBED_LOOKUP_TABLE 1
 #define QMBED_LOOKUP_SEARCH 2
@@ -350,7 +350,7 @@ QMBED_API int qmbed_gpu_scan_solve(int n_sectors, int n_components, const qmbed_
  * block fewer than it waits for; *status receives 1 when the bounded spin
  * ended in the time-out status (the kernel returns instead of hanging). */
 QMBED_API int qmbed_gpu_scan_barrier_selftest(int device, int* status);
-/* Test of the multi-pass flip-chain action's bounded wait on its box copies
+/* Test of the flip-chain box action's bounded wait on its box copies
  * (no reference counterpart): a barrier armed for bytes that no copy
  * delivers is polled 1024 times; *status receives 1 when the wait gave up
  * (the kernel returns instead of hanging). */

@@ -5,7 +5,7 @@
 // spectrum (Tal-Ezer and Kosloff, J. Chem. Phys. 81, 3967 (1984)). The sum is
 // evaluated by the Clenshaw recurrence b_k = c_k psi + 2 Ht b_{k+1} - b_{k+2},
 // f = c_0 psi + Ht b_1 - b_2, so no accumulator vector is read or written:
-// each step is one fused flip-chain application (two tiled passes) that reads
+// each step is one fused flip-chain application (TMA boxes) that reads
 // b_{k+1}, b_{k+2} and psi and writes b_k over b_{k+2}.
 #include <algorithm>
 #include <cmath>
@@ -148,7 +148,7 @@ void chebyshev_run(const SpinOperator& op, const double* initial, cudaMemcpyKind
     emit(t);
   }
   ops.sync();
-  fc->check_status();  // a multi-pass box wait that timed out
+  fc->check_status();  // a box wait that timed out
 }
 
 }  // namespace

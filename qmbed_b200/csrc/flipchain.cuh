@@ -30,7 +30,7 @@ struct FlipStep {
   double kappa_re = 0.0, kappa_im = 0.0;
 };
 
-// Runs the multi-pass action's bounded stage wait on a barrier that no copy
+// Runs the box action's bounded wait on a barrier that no copy
 // completes (1024 polls) on `device`; returns 1 when it gave up as designed.
 int flip_stage_wait_selftest(int device);
 
@@ -54,7 +54,7 @@ class FlipChain {
              cudaStream_t stream) const;
   // Gershgorin-type bounds: |D| max over the diagonal terms plus sum |x|.
   double norm_bound() const;
-  // Raises when a multi-pass launch recorded a timed-out tile wait (and clears it).
+  // Raises when a box launch recorded a timed-out wait (and clears it).
   void check_status() const;
 
  private:

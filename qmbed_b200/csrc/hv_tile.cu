@@ -1838,7 +1838,9 @@ void launch_hop_kernel(const HopArgs& a, size_t smem, cudaStream_t stream) {
   QMBED_LAUNCH_CHECK();
 }
 
-// The hop kernel serves chain programs whose only off-diagonal class is the
+// Blocks of vectors, and single vectors that launch_exchange() declines (chains
+// of fewer than five sites, tables beyond 2^32 entries): the hop kernel serves
+// chain programs whose only off-diagonal class is the
 // nearest-neighbour bond, on real fixed-weight sectors whose image table has
 // 32-bit entries without a phase index.
 bool hop_form(const SpinBasis& basis, const DeviceFlipProgram& prog, const ImageTable* table) {

@@ -108,7 +108,7 @@ bool hermitian_by_terms(const std::vector<Instance>& adjoint, const std::vector<
                         const LocalFactors& f, int sites);
 
 // kLookupTableGeneric: the image table with the general tile kernel even
-// where the nearest-neighbour hop kernel applies (kept for comparisons).
+// where the exchange or hop kernel applies (kept for comparisons).
 enum LookupMode : int { kLookupAuto = 0, kLookupTable = 1, kLookupSearch = 2, kLookupLegacy = 3,
                         kLookupTableGeneric = 4 };
 

@@ -530,10 +530,14 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
 // Block action on tiles: a row's NB values are LPR consecutive 16-byte
 // vectors, one per lane, and a warp takes 32 / LPR rows of a tile (LPR
 // neighbouring warps share one). Entries are read once per row and shared by
-// its lanes. Bound by the L2: every gathered column is 32 to 128 bytes, and at
-// 32 sites (9,398,520 rows, FP32, 8 columns) the 634 us move 6.6 GB through it
-// (10.4 TB/s); the row lists took 766 us. At 28 sites (718,146 rows, 16
-// columns) 70 against 75 us in FP32 and 138 against 139 us in FP64.
+// its lanes. Bound by the L1's data path (75% at 28 sites, 16 columns FP32: each
+// gathered column is 32 to 128 bytes of a line of its own) and by the L2: at 32
+// sites (9,398,520 rows, FP32, 8 columns) the 589 us move 6.6 GB through it
+// (11 TB/s); the row lists took 766 us. At 34 sites it is DRAM: 16.1 GB in 2.65 ms,
+// where the row lists moved 24.5 GB in 4.24. At 28 sites (718,146 rows, 16 columns) 70
+// against 75 us in FP32 and 136 against 139 us in FP64. Many small blocks in one
+// moving window of rows are what is fast: blocks of 256 to 1024 threads with
+// chunks of rows of their own, for reuse in the L1, took 1.2 to 1.9 times as long.
 template <typename T, int NB, bool HAS_P, int KB>
 __global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
                                                          const uint32_t* __restrict__ entries, int col_bits,
