@@ -431,6 +431,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
   int l = 0;
   int retained = 0;
   bool retained_actions = false;
+  std::vector<double> retained_norms;  // of the retained columns where the candidates' launch took them
   for (int i = 0; i < n_initial; ++i) c.copy(initial->col(i), RC.col(i));
   retained = n_initial;
   size_t iterations = 0, passes = 0, seconds = 0;
@@ -442,7 +443,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
     for (int i = 0; i < retained; ++i) {
       void* slot = Q.col(l + b);
       if (reuse) {
-        const double norm = c.norm(RC.col(i));
+        const double norm = i < static_cast<int>(retained_norms.size()) ? retained_norms[i] : c.norm(RC.col(i));
         if (std::isfinite(norm) && norm > 1.0e-14) {
           c.ops.scale_into(RC.col(i), slot, n, norm, c.prec, c.cplx);
           c.ops.scale_into(RCA.col(i), W.col(a), n, norm, c.prec, c.cplx);
@@ -557,7 +558,16 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
     c.ops.combine(Q.col(l), n, size, Y.data(), K, C.col(0), n, n, c.prec, c.cplx);
     c.ops.combine(W.col(0), n, size, Y.data(), K, CA.col(0), n, n, c.prec, c.cplx);
     std::vector<Candidate> candidates;
+    std::vector<BlockOps::RitzCandidate> ritz;
+    if (c.prec != 64 || !c.ops.ritz_candidates(static_cast<double*>(C.col(0)), static_cast<double*>(CA.col(0)), n, K,
+                                               c.cplx, ritz))
+      ritz.clear();
     for (int kk = 0; kk < K; ++kk) {
+      if (!ritz.empty()) {
+        if (!std::isfinite(ritz[kk].norm) || ritz[kk].norm <= kEps) nonconvergence(iterations, ritz[kk].norm);
+        candidates.push_back({ritz[kk].value, ritz[kk].residual, kk});
+        continue;
+      }
       const double norm = c.norm(C.col(kk));
       if (!std::isfinite(norm) || norm <= kEps) nonconvergence(iterations, norm);
       c.scale(C.col(kk), norm);
@@ -572,6 +582,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
     last_residual = 0.0;
     for (int i = 0; i < static_cast<int>(candidates.size()) && i < active; ++i)
       last_residual = std::max(last_residual, candidates[i].residual);
+    retained_norms.clear();
     // Lock converged pairs, retain the rest (with their actions) in rank order.
     int next = 0;
     for (int rank = 0; rank < static_cast<int>(candidates.size()); ++rank) {
@@ -589,6 +600,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
       } else if (next < keep) {
         c.copy(C.col(cand.slot), RC.col(next));
         c.copy(CA.col(cand.slot), RCA.col(next));
+        if (!ritz.empty()) retained_norms.push_back(ritz[cand.slot].norm_after);
         ++next;
       }
     }

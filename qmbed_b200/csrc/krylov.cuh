@@ -88,6 +88,14 @@ class BlockOps {
   // unnormalised, real part only; imaginary parts zero for complex vectors.
   void lcg_start(void* out, uint64_t n, uint64_t seed, int precision, bool cplx);
   // r = y - lambda x; returns ||r||  (FP64 accumulation).
+  // Normalises `count` Ritz candidates (columns of C, FP64) and their actions
+  // (CA) in one launch and reads their norms before, Ritz values, residual
+  // norms and norms after. False, with nothing done, for columns too long for
+  // one block each.
+  struct RitzCandidate {
+    double norm, value, residual, norm_after;
+  };
+  bool ritz_candidates(double* C, double* CA, uint64_t n, int count, bool cplx, std::vector<RitzCandidate>& out);
   double residual_norm(const void* y, const void* x, double lambda, uint64_t n, int precision, bool cplx);
   void sync();
 
