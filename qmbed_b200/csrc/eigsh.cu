@@ -289,7 +289,8 @@ EigshResult lanczos_window(Ctx& c, const EigshOptions& o, const void* initial_de
     size_t it = begin;
     for (; it < end && !finished; ++it) {
       const OrthoRecord& r = records[it - begin];
-      if (r.second && !whole) break;  // redone below from this step on
+      // redone below from this step on: a second pass is due, or the next column was not written (norms that are not finite)
+      if ((r.second && !whole) || (!r.ok && !(r.norm <= 1.0e-14))) break;
       alphas.push_back(r.h.back().real());
       size = it + 1;
       passes += r.second ? 2 : 1;

@@ -142,8 +142,10 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   std::vector<double> betas;
   double previous_beta = 0.0;
   // Steps queue up to kQueuedSteps at a time (no host round trip between
-  // them); one that needs a second pass the queue does not make is redone by
-  // the loop below, which then goes on step by step to the next queue.
+  // them); one that needs a second pass the queue does not make, or whose next
+  // column it did not write although the run goes on (norms up to the kernels'
+  // 1e-14 that are above the tolerance), is redone by the loop below, which
+  // then goes on step by step to the next queue.
   bool finished = false;
   for (int index = 0; index < capacity && !finished; ++index) {
     {
@@ -160,7 +162,7 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
       int i = index;
       for (; i < end && !finished; ++i) {
         const OrthoRecord& r = records[static_cast<size_t>(i - index)];
-        if (r.second && !whole) break;
+        if ((r.second && !whole) || (!r.ok && r.norm > tolerance)) break;
         ++d.applications;
         if (std::fabs(r.h.back().imag()) > std::max(tolerance, 1.0e-10)) raise(QMBED_NON_HERMITIAN, "");
         if (r.second) ++d.second_passes;
