@@ -1908,6 +1908,30 @@ bool launch_hop(const SpinBasis& basis, const DeviceFlipProgram& prog, const Ima
   return true;
 }
 
+template <typename T, typename S, bool CV, bool CC, bool D2, bool HOLES, int U>
+void launch_exchange_kernel(const ExchangeArgs& a, size_t smem, cudaStream_t stream) {
+  auto kernel = exchange_row_kernel<T, S, CV, CC, D2, HOLES, U>;
+  // resident blocks per SM for this instantiation, cached per (device, smem):
+  // the variants' kernels are all of one type, so the cache belongs to a
+  // function template (a generic lambda's would be one for all of them)
+  static thread_local int cached_device = -1, cached_sms = 0, cached_per_sm = 0;
+  static thread_local size_t cached_smem = 0;
+  int device = 0;
+  QMBED_CUDA(cudaGetDevice(&device));
+  if (cached_device != device || cached_smem != smem) {
+    if (smem > 48 * 1024)
+      QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    QMBED_CUDA(cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, device));
+    QMBED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, kernel, kExchangeThreads, smem));
+    cached_device = device;
+    cached_smem = smem;
+  }
+  const uint64_t needed = (a.rows + kExchangeThreads - 1) / kExchangeThreads;
+  const uint64_t cap = static_cast<uint64_t>(cached_sms) * std::max(cached_per_sm, 1);
+  launch_dependent(kernel, static_cast<unsigned>(std::min(needed, cap)), kExchangeThreads, smem, stream, a);
+  QMBED_LAUNCH_CHECK();
+}
+
 // The exchange kernel serves single vectors of chain programs that exchange
 // neighbours or next-nearest neighbours with one real amplitude per class
 // (Heisenberg, XXZ, J1-J2), on fixed-weight sectors with a 32-bit image table
@@ -1967,33 +1991,15 @@ bool launch_exchange(const SpinBasis& basis, const DeviceFlipProgram& prog, cons
   // (620 MB) 129 against 137 us in FP32, 33 sites (4.7 GB) 1071 against 1382;
   // 28 sites (160 MB) 39.6 against 37.4.
   const bool far = table->bytes >= (512ull << 20);
-  auto run = [&](auto kernel) {
-    static thread_local int cached_device = -1, cached_sms = 0, cached_per_sm = 0;
-    static thread_local size_t cached_smem = 0;
-    int device = 0;
-    QMBED_CUDA(cudaGetDevice(&device));
-    if (cached_device != device || cached_smem != smem) {
-      if (smem > 48 * 1024)
-        QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      QMBED_CUDA(cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, device));
-      QMBED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, kernel, kExchangeThreads, smem));
-      cached_device = device;
-      cached_smem = smem;
-    }
-    const uint64_t needed = (a.rows + kExchangeThreads - 1) / kExchangeThreads;
-    const uint64_t cap = static_cast<uint64_t>(cached_sms) * std::max(cached_per_sm, 1);
-    launch_dependent(kernel, static_cast<unsigned>(std::min(needed, cap)), kExchangeThreads, smem, l.stream, a);
-    QMBED_LAUNCH_CHECK();
-  };
   auto by_holes = [&](auto t, auto st, auto c1, auto c2, auto c3) {
     using T = decltype(t);
     using S = decltype(st);
     constexpr bool V1 = decltype(c1)::value, V2 = decltype(c2)::value, V3 = decltype(c3)::value;
     constexpr int kFar = kExchangeMaxStep;
-    if (holes) far ? run(exchange_row_kernel<T, S, V1, V2, V3, true, kFar>)
-                   : run(exchange_row_kernel<T, S, V1, V2, V3, true, 4>);
-    else far ? run(exchange_row_kernel<T, S, V1, V2, V3, false, kFar>)
-             : run(exchange_row_kernel<T, S, V1, V2, V3, false, 4>);
+    if (holes) far ? launch_exchange_kernel<T, S, V1, V2, V3, true, kFar>(a, smem, l.stream)
+                   : launch_exchange_kernel<T, S, V1, V2, V3, true, 4>(a, smem, l.stream);
+    else far ? launch_exchange_kernel<T, S, V1, V2, V3, false, kFar>(a, smem, l.stream)
+             : launch_exchange_kernel<T, S, V1, V2, V3, false, 4>(a, smem, l.stream);
   };
   auto by_d2 = [&](auto t, auto st, auto c1, auto c2) {
     if (d2) by_holes(t, st, c1, c2, std::true_type{});
