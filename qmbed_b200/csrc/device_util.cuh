@@ -7,12 +7,19 @@ namespace qmbed {
 
 constexpr int kBinomStride = 129;  // binomial table is [n][k], n,k <= 128
 
-// 16-byte vector access to rows of row-major blocks (addresses 16-byte aligned).
-// First statement of a kernel that launch_dependent() may start while its
+// First call of a kernel that launch_dependent() may start while its
 // predecessor in the stream drains: waits until that one has completed and its
-// writes are visible, then lets the next such launch follow. Nothing but the
-// launch's own arguments may be read before it. What the predecessor wrote is
-// read with __ldcg: the non-coherent path asks for data constant over the launch.
+// writes are visible, then lets the next such launch follow.
+//
+// In front of it a kernel may read what was complete before the launch was
+// issued and nothing writes any more: its arguments, and an operator's own rows
+// and tables (its constructor waits for them). Behind it, what the predecessor
+// writes (the vector a product acts on, partial sums, a record) takes ordinary
+// loads, or __ldcg: the grid is there while the predecessor still writes, and
+// the non-coherent path (__ldg, ld.global.nc, const __restrict__ pointers)
+// promises data constant over the grid's life. Data of earlier launches is
+// constant then: each of them waited for the one before it, or was launched
+// without overlap.
 __device__ __forceinline__ void await_previous() {
 #if __CUDA_ARCH__ >= 900
   cudaGridDependencySynchronize();
@@ -41,8 +48,10 @@ void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, siz
   QMBED_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...));
 }
 
-// load16 reads through the read-only path: only for data no thread of the
-// launch writes. load16_rw is the coherent form for rows a launch rewrites.
+// 16-byte vector access to rows of row-major blocks (addresses 16-byte
+// aligned). load16 reads through the read-only path: only for data constant
+// over the launch. load16_rw is the coherent form, for rows that the launch
+// rewrites and for the predecessor's output in a dependent launch.
 __device__ __forceinline__ void load16(const float* p, float (&v)[4]) {
   const float4 t = __ldg(reinterpret_cast<const float4*>(p));
   v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;

@@ -1213,7 +1213,9 @@ struct ExchangeElem<double, true> {
 };
 
 // Loads of the lanes where `on` holds, zero in the others, without a branch:
-// the loads of one step all issue before the first is waited for.
+// the loads of one step all issue before the first is waited for. Table
+// entries are constant; vector elements may come from the launch before
+// (ordinary loads, see await_previous).
 __device__ __forceinline__ uint32_t load_if(bool on, const uint32_t* p) {
   uint32_t v;
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
@@ -1223,7 +1225,7 @@ __device__ __forceinline__ uint32_t load_if(bool on, const uint32_t* p) {
 }
 __device__ __forceinline__ float load_if(bool on, const float* p) {
   float v;
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.f32 %0, [%1];\n\t}"
                : "=f"(v)
                : "l"(p), "r"(static_cast<uint32_t>(on)));
   return v;
@@ -1231,7 +1233,7 @@ __device__ __forceinline__ float load_if(bool on, const float* p) {
 __device__ __forceinline__ double load_if(bool on, const double* p) {
   double v;
   asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t@q ld.global.nc.f64 %0, [%1];\n\t}"
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t@q ld.global.f64 %0, [%1];\n\t}"
       : "=d"(v)
       : "l"(p), "r"(static_cast<uint32_t>(on)));
   return v;
@@ -1240,7 +1242,7 @@ __device__ __forceinline__ float2 load_if(bool on, const float2* p) {
   float2 v;
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
-      "@q ld.global.nc.v2.f32 {%0, %1}, [%2];\n\t}"
+      "@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
       : "=f"(v.x), "=f"(v.y)
       : "l"(p), "r"(static_cast<uint32_t>(on)));
   return v;
@@ -1249,7 +1251,7 @@ __device__ __forceinline__ double2 load_if(bool on, const double2* p) {
   double2 v;
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\tmov.f64 %1, 0d0000000000000000;\n\t"
-      "@q ld.global.nc.v2.f64 {%0, %1}, [%2];\n\t}"
+      "@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
       : "=d"(v.x), "=d"(v.y)
       : "l"(p), "r"(static_cast<uint32_t>(on)));
   return v;
@@ -1358,7 +1360,7 @@ __global__ void __launch_bounds__(kExchangeThreads) exchange_row_kernel(const __
     // an entry outside the sector reads nothing; its value index is taken as 0
     auto take = [&](int cls, uint32_t e) {
       if (HOLES && e == 0xffffffffu) return;
-      add(cls, e, __ldg(x + (e & col_mask)));
+      add(cls, e, x[e & col_mask]);
     };
     S h1 = (s ^ (s >> 1)) & static_cast<S>(a.bonds[0]);
     S h2 = D2 ? (s ^ (s >> 2)) & static_cast<S>(a.bonds[1]) : 0;

@@ -65,8 +65,8 @@ __device__ inline double warp_sum(double v) {
 constexpr int kMaxSlab = 2048;
 template <bool CPLX>
 __global__ void __launch_bounds__(kThreads) panel_dot_kernel(const double* __restrict__ A, uint64_t ld, int m,
-                                                             const double* __restrict__ w, uint64_t n, int slab,
-                                                             int keep, double* __restrict__ partials) {
+                                                             const double* w, uint64_t n, int slab, int keep,
+                                                             double* __restrict__ partials) {
   constexpr int W = CPLX ? 2 : 1;
   extern __shared__ __align__(16) double ws[];
   const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * slab;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) multi_dot_kernel(const T* __restrict
 // out[t] = sum_b partials[(t/2 * G + b) * 2 + t%2]: one block per output,
 // strided per-thread sums then a shared-memory tree, both in a fixed order.
 constexpr int kFinishThreads = 128;
-__global__ void __launch_bounds__(kFinishThreads) finish_kernel(const double* __restrict__ partials, int G, int count,
+__global__ void __launch_bounds__(kFinishThreads) finish_kernel(const double* partials, int G, int count,
                                                                 double* __restrict__ out) {
   const int t = blockIdx.x;
   await_previous();
@@ -988,8 +988,8 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 enum { kReal = 0, kRealPair = 1, kComplex = 2 };
 template <int MODE, int ROWS>
 __global__ void __launch_bounds__(kOrthoThreads, 4) orthogonalize_kernel(const double* __restrict__ Q, uint64_t n, int m,
-                                                                      const double* __restrict__ h, double beta_value,
-                                                                      const double* __restrict__ beta_device,
+                                                                      const double* h, double beta_value,
+                                                                      const double* beta_device,
                                                                       int before_mode, int keep, const double* src,
                                                                       double* w, double* __restrict__ partials) {
   extern __shared__ double hs[];
@@ -1156,10 +1156,9 @@ __global__ void __launch_bounds__(128) orthogonalize_finish_kernel(const double*
 // the first writes the record (norms before and after, the DGKS verdict and the
 // last overlap), all scale the vector into the next column. One launch; a
 // record kernel of its own took 3.2 us and a gap in front of the scaling.
-__global__ void __launch_bounds__(kThreads) scale_and_record_kernel(const double* __restrict__ partials, int G, int m,
-                                                                    const double* __restrict__ h,
-                                                                    double* __restrict__ record,
-                                                                    const double* __restrict__ src,
+__global__ void __launch_bounds__(kThreads) scale_and_record_kernel(const double* partials, int G, int m,
+                                                                    const double* h, double* __restrict__ record,
+                                                                    const double* src,
                                                                     double* __restrict__ dst, uint64_t count) {
   __shared__ double tree[2][128];
   await_previous();

@@ -371,14 +371,15 @@ struct Pair2<double> {
   using type = double2;
 };
 
-// Complex element i: one 8/16-byte load when the vector allows it (VEC2).
+// Complex element i of a product's input (an ordinary load, see
+// await_previous): 8 or 16 bytes at once when the vector allows it (VEC2).
 template <typename T, bool VEC2>
 __device__ __forceinline__ typename Pair2<T>::type load_complex(const T* x, uint64_t i) {
   using P = typename Pair2<T>::type;
-  if (VEC2) return __ldg(reinterpret_cast<const P*>(x) + i);
+  if (VEC2) return reinterpret_cast<const P*>(x)[i];
   P v;
-  v.x = __ldg(x + 2 * i);
-  v.y = __ldg(x + 2 * i + 1);
+  v.x = x[2 * i];
+  v.y = x[2 * i + 1];
   return v;
 }
 
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
                                                          const T* __restrict__ diag,
                                                          const uint16_t* __restrict__ orbits,
                                                          const double* __restrict__ sqrt_table,
-                                                         const T* __restrict__ x, T* __restrict__ y) {
+                                                         const T* x, T* y) {
   using P = typename Pair2<T>::type;
   using V = typename std::conditional<VALC, P, T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
       xr = v.x;
       xi = v.y;
     } else {
-      xr = __ldg(x + r);
+      xr = x[r];
     }
   }
   __syncthreads();
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(kSpmvThreads) tile_spmv_kernel(uint64_t n, con
         gr[u] = v.x;
         gi[u] = v.y;
       } else {
-        gr[u] = __ldg(x + (e[u] & col_mask));
+        gr[u] = x[e[u] & col_mask];
       }
     }
     uint32_t f[KB];
@@ -542,7 +543,7 @@ template <typename T, int NB, bool HAS_P, int KB>
 __global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32_t* __restrict__ tile_ptr,
                                                          const uint32_t* __restrict__ entries, int col_bits,
                                                          const double2* __restrict__ values, int codes,
-                                                         const T* __restrict__ diag, const T* __restrict__ z,
+                                                         const T* __restrict__ diag, const T* z,
                                                          const T* p, T* out, T alpha, T beta, T gamma) {
   constexpr int VEC = 16 / sizeof(T);
   constexpr int LPR = NB / VEC;
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32
 #pragma unroll
     for (int u = 0; u < KB; ++u) {
       if (e[u] != kNoEntry) {
-        load16(z + static_cast<uint64_t>(e[u] & col_mask) * NB + part * VEC, g[u]);
+        load16_rw(z + static_cast<uint64_t>(e[u] & col_mask) * NB + part * VEC, g[u]);
       } else {
 #pragma unroll
         for (int v = 0; v < VEC; ++v) g[u][v] = 0;
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(256) tile_spmm_kernel(uint64_t n, const uint32
   }
   const T d = __ldcs(diag + r);
   T self[VEC], o[VEC];
-  load16(z + r * NB + part * VEC, self);
+  load16_rw(z + r * NB + part * VEC, self);
 #pragma unroll
   for (int v = 0; v < VEC; ++v) o[v] = alpha * (acc[v] + d * self[v]) + beta * self[v];
   if (HAS_P) {
