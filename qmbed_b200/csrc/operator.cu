@@ -1274,8 +1274,21 @@ void SpinOperator::assemble_row_lists() {
   assembly_seconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
 }
 
+namespace {
+
+bool overlap(const void* a, const void* b, size_t bytes) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+  return p < q + bytes && q < p + bytes;
+}
+
+}  // namespace
+
+size_t SpinOperator::vector_bytes(int precision, bool complex_vectors) const {
+  return static_cast<size_t>(dim()) * (complex_vectors ? 2 : 1) * (precision == kFP64 ? 8 : 4);
+}
+
 void SpinOperator::ensure_scratch(int precision, bool complex_vectors) const {
-  const size_t bytes = static_cast<size_t>(dim()) * (complex_vectors ? 2 : 1) * (precision == kFP64 ? 8 : 4);
+  const size_t bytes = vector_bytes(precision, complex_vectors);
   if (scaled_bytes_ < bytes) {
     scaled_x_.allocate(bytes);
     scaled_bytes_ = bytes;
@@ -1331,7 +1344,15 @@ void SpinOperator::apply(int precision, bool complex_vectors, const void* x, voi
   }
   // Stored rows.
   if (tile_) {
-    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, x, y, stream);
+    // symmetry sectors take y over x, as with row lists (whose input is scaled into a buffer of its own)
+    const size_t bytes = vector_bytes(precision, cplx);
+    const void* from = x;
+    if (basis_->symmetric() && overlap(x, y, bytes)) {
+      ensure_scratch(precision, cplx);
+      QMBED_CUDA(cudaMemcpyAsync(scaled_x_.get(), x, bytes, cudaMemcpyDeviceToDevice, stream));
+      from = scaled_x_.get();
+    }
+    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, from, y, stream);
     return;
   }
   const bool scaled = basis_->symmetric();
@@ -1421,13 +1442,18 @@ void SpinOperator::apply_with_scratch(int precision, bool complex_vectors, const
   }
   if (!real_ && !cplx) raise(QMBED_UNSUPPORTED_BACKEND, "real action requires an operator with real-valued storage");
   const int comps = cplx ? 2 : 1;
-  const size_t need = static_cast<size_t>(n) * comps * (precision == kFP64 ? 8 : 4);
+  const size_t need = vector_bytes(precision, cplx);
   if (need > scratch_bytes)
     raise(QMBED_DIMENSION_MISMATCH, "symmetry sectors with stored rows take vectors of at most " +
                                         std::to_string(scratch_bytes) + " bytes here; this one has " +
                                         std::to_string(need));
-  if (tile_) {  // needs no scaled vector
-    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, x, y, stream);
+  if (tile_) {  // needs no scaled vector, only the input out of the output's way
+    const void* from = x;
+    if (overlap(x, y, need)) {
+      QMBED_CUDA(cudaMemcpyAsync(scratch, x, need, cudaMemcpyDeviceToDevice, stream));
+      from = scratch;
+    }
+    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, from, y, stream);
     return;
   }
   {

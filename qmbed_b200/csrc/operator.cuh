@@ -167,6 +167,7 @@ class SpinOperator {
   void build_instances(const std::vector<TermDesc>& terms, const OperatorChecks& checks);
   void assemble();
   void assemble_row_lists();
+  size_t vector_bytes(int precision, bool complex_vectors) const;
   void ensure_scratch(int precision, bool complex_vectors) const;
   void launch_block_matrix_free(int precision, int nb, const void* z, const void* p, void* out, double alpha,
                                 double beta, double gamma, cudaStream_t stream) const;
