@@ -1198,6 +1198,7 @@ struct ExchangeArgs {
 
 constexpr int kExchangeThreads = 128;
 constexpr int kExchangeMaxStep = 8;  // sites of a step at most
+constexpr int kExchangeMaxSmem = 96 * 1024;
 
 template <typename T, bool CV>
 struct ExchangeElem {
@@ -1921,8 +1922,9 @@ void launch_exchange_kernel(const ExchangeArgs& a, size_t smem, cudaStream_t str
   int device = 0;
   QMBED_CUDA(cudaGetDevice(&device));
   if (cached_device != device || cached_smem != smem) {
-    if (smem > 48 * 1024)
-      QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // one limit for every size: the attribute belongs to the kernel, and other
+    // threads launch it with sizes of their own
+    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExchangeMaxSmem));
     QMBED_CUDA(cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, device));
     QMBED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, kernel, kExchangeThreads, smem));
     cached_device = device;
@@ -1964,7 +1966,7 @@ bool launch_exchange(const SpinBasis& basis, const DeviceFlipProgram& prog, cons
   const size_t value = static_cast<size_t>(l.precision == 64 ? 8 : 4) * (cc ? 2 : 1);
   const size_t smem = (value << code_bits) + cells * 4 * (d2 ? 6 : 2) +
                       static_cast<size_t>(basis.rank_chunk_count()) * kRankChunkValues * basis.rank_chunk_stride() * 4;
-  if (smem > 96 * 1024) return false;
+  if (smem > static_cast<size_t>(kExchangeMaxSmem)) return false;
   a.dim = basis.dim();
   a.row0 = l.row0;
   a.rows = std::min(l.rows, a.dim - std::min(l.row0, a.dim));

@@ -1576,8 +1576,8 @@ void device_hermitian_eigen(int n, const std::vector<C64>& a, std::vector<double
     const int items = half * half, trips = (items + kJacobiBlockItems - 1) / kJacobiBlockItems;
     const int threads = ((items + trips - 1) / trips + 31) / 32 * 32 + (half + 31) / 32 * 32;
     auto kernel = real ? jacobi_smem_kernel<false> : jacobi_smem_kernel<true>;
-    if (smem > 48 * 1024)
-      QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // one limit for every size: handles are solved on several threads
+    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kJacobiMaxSmem)));
     kernel<<<1, threads, smem, stream>>>(n, buf, buf + first, buf + first + nv, 100);
     QMBED_LAUNCH_CHECK();
     QMBED_CUDA(cudaMemcpyAsync(host.data(), buf + first, (nn * w + nv) * sizeof(double), cudaMemcpyDeviceToHost, stream));

@@ -26,6 +26,7 @@ constexpr int kMaxRowSlots = 64;
 constexpr int kMaxTableCodes = 2048;
 constexpr int kMaxStoredValues = 1024;  // distinct values of a packed real operator
 constexpr int kFillThreads = 256;
+constexpr int kMaxProgramSmem = 96 * 1024;  // products and fence keys in shared memory
 constexpr int kSumSlots = 4096;  // dictionary of coalesced values (open addressing)
 
 // One off-diagonal site pair on the device.
@@ -766,7 +767,7 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
   a.used = reinterpret_cast<unsigned int*>(base + scratch + 16 + kSumSlots * 8);
   const size_t program_smem = groups.size() * sizeof(RowGroup) + pairs.size() * sizeof(RowPair) +
                               static_cast<size_t>(a.n_fences) * 8;
-  if (program_smem > 96 * 1024) return false;
+  if (program_smem > static_cast<size_t>(kMaxProgramSmem)) return false;
   const int sms = device_sms(basis.device());
   const size_t group_smem = groups.size() * sizeof(RowGroup);
   const unsigned wgrid = static_cast<unsigned>(std::min<uint64_t>((tiles + 7) / 8, static_cast<uint64_t>(sms) * 8));
@@ -794,8 +795,9 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
   const bool shift = p.has_momentum && p.momentum != 0;
   auto kernel = p.sites <= 32 ? (shift ? tile_fill_kernel<uint32_t, true> : tile_fill_kernel<uint32_t, false>)
                               : (shift ? tile_fill_kernel<uint64_t, true> : tile_fill_kernel<uint64_t, false>);
-  if (smem > 48 * 1024)
-    QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  // one limit for every size: operators may be assembled on several threads
+  QMBED_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kMaxProgramSmem + kFillThreads / 32 * kMaxRowSlots * 128));
   int per_sm = 1;
   QMBED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFillThreads, smem));
   const unsigned grid = static_cast<unsigned>(
