@@ -148,7 +148,6 @@ void chebyshev_run(const SpinOperator& op, const double* initial, cudaMemcpyKind
     emit(t);
   }
   ops.sync();
-  fc->check_status();  // a box wait that timed out
 }
 
 }  // namespace

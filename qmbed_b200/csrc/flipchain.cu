@@ -253,8 +253,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 // Bounded wait for the phase `parity` of a stage barrier; false on time-out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (unsigned polls = 0; polls < kWaitPolls; ++polls)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned limit = kWaitPolls) {
+  for (unsigned polls = 0; polls < limit; ++polls)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
@@ -318,6 +318,18 @@ __device__ __forceinline__ void axpy(Word<float>& acc, unsigned long long c, con
 __device__ __forceinline__ void axpy(Word<double>& acc, double c, const Word<double>& v) {
   acc.a = fma(c, v.a, acc.a);
   acc.b = fma(c, v.b, acc.b);
+}
+// A box (or a part of it) whose copy did not arrive within the wait: the thread
+// that gave up writes words `first` .. `first + count - 1` itself, from ordinary
+// loads. The copy may still be under way; it brings the same bytes, and the
+// second wait keeps the block from ending in front of it. Word v of the box is
+// word base | (v below run_bits) | (v above them) << shift of x.
+template <typename W>
+__device__ __noinline__ void fill_words(W* box, const W* x, int first, int count, uint64_t base, int run_bits, int shift,
+                                        uint64_t* bar) {
+  for (int v = first; v < first + count; ++v)
+    box[v] = x[base | static_cast<uint64_t>(v & ((1 << run_bits) - 1)) | (static_cast<uint64_t>(v >> run_bits) << shift)];
+  mbar_wait(bar, 0);
 }
 __device__ __forceinline__ Word<float> load_word(const Word<float>* p) {
   const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
@@ -406,7 +418,7 @@ struct BoxArgs {
   const Word<T>* q;
   double alpha, beta;
   T gamma, kr, ki;
-  int* status;
+  unsigned polls;  // limit of a wait on a copy
 };
 
 constexpr int kRegBits = 3;  // a thread's eight words differ in the top bits of the box
@@ -481,13 +493,13 @@ struct BoxDiagonal {
 // starts with the first eighth that arrives, and sum j is complete after
 // eighth max(j, j ^ 4). GROUP: only the flips along word bits >= a.lo.
 template <typename T, bool CPLX, int VB, bool GROUP, typename Wait, typename Own>
-__device__ __forceinline__ bool box_flips(const BoxArgs<T>& a, const Word<T>* box, int v0, Wait&& wait, Own&& own_part,
+__device__ __forceinline__ void box_flips(const BoxArgs<T>& a, const Word<T>* box, int v0, Wait&& wait, Own&& own_part,
                                           Word<T> (&acc)[kWordsPerThread]) {
   constexpr int VBITS = WordShape<T, CPLX>::VBITS;
   constexpr int LOW = VB - kRegBits;
 #pragma unroll
   for (int j = 0; j < kWordsPerThread; ++j) {
-    if (!wait(j)) return false;
+    wait(j);
     const int v = v0 | (j << LOW);
     const Word<T> own = load_word(box + v);
     if (!GROUP) {
@@ -502,7 +514,6 @@ __device__ __forceinline__ bool box_flips(const BoxArgs<T>& a, const Word<T>* bo
     for (int i = 0; i < LOW; ++i)
       if (!GROUP || i >= a.lo) axpy(acc[j], a.cbit[i], load_word(box + (v ^ (1 << i))));
   }
-  return true;
 }
 
 // A block per contiguous box of 2^VB words (8 or 10), the flips of the `extra`
@@ -551,14 +562,13 @@ __global__ void __launch_bounds__((1 << VB) / kWordsPerThread) flip_box_kernel(c
   };
   if (FAR_FIRST) far_flips();
   const BoxDiagonal<T, CPLX, VB> diagonal(a);
-  if (!box_flips<T, CPLX, VB, false>(
-          a, box, static_cast<int>(threadIdx.x), [&](int j) { return j > 0 || mbar_wait(&full, 0); },
-          [&](int v, const W& own, W& sum) { diagonal.add(a, gbase, dword, v, own, sum); }, acc)) {
-    // the copy may still be in flight: one more bounded wait before the box is given up
-    atomicExch(a.status, 1);
-    mbar_wait(&full, 0);
-    return;
-  }
+  box_flips<T, CPLX, VB, false>(
+      a, box, static_cast<int>(threadIdx.x),
+      [&](int j) {
+        if (j == 0 && !mbar_wait(&full, 0, a.polls))
+          fill_words(box, a.x, 0, 1 << VB, gbase, VB, 0, &full);
+      },
+      [&](int v, const W& own, W& sum) { diagonal.add(a, gbase, dword, v, own, sum); }, acc);
   if (!FAR_FIRST) far_flips();
 #pragma unroll
   for (int j = 0; j < kWordsPerThread; ++j) {
@@ -616,13 +626,13 @@ __global__ void __launch_bounds__(kPassThreads, 3) flip_group_kernel(const __gri
       before[j] = load_early(a.out + global_word(v0 | (j << LOW)));
       acc[j].a = acc[j].b = 0;
     }
-    if (!box_flips<T, CPLX, VB, true>(
-            a, box, v0, [&](int j) { return trip > 0 || mbar_wait(&full[j], 0); }, [](int, const W&, W&) {}, acc)) {
-      // copies may still be in flight: one more bounded wait for each before the box is given up
-      atomicExch(a.status, 1);
-      for (int j = 0; j < kWordsPerThread; ++j) mbar_wait(&full[j], 0);
-      return;
-    }
+    box_flips<T, CPLX, VB, true>(
+        a, box, v0,
+        [&](int j) {
+          if (trip == 0 && !mbar_wait(&full[j], 0, a.polls))
+            fill_words(box, a.x, j << LOW, 1 << LOW, gbase, run_bits, a.b0 - VBITS, &full[j]);
+        },
+        [](int, const W&, W&) {}, acc);
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; ++j) {
       axpy(acc[j], coef_of(static_cast<T>(1)), before[j]);
@@ -633,7 +643,7 @@ __global__ void __launch_bounds__(kPassThreads, 3) flip_group_kernel(const __gri
 
 // Self-test of the bounded stage wait: one thread arms an mbarrier for bytes
 // that no copy will deliver and waits `polls` times; status receives 1 when
-// the wait gave up (the kernel then returns as the passes do).
+// the wait gave up.
 __global__ void stage_wait_selftest_kernel(unsigned polls, int* status) {
   __shared__ __align__(8) uint64_t bar;
   if (threadIdx.x != 0) return;
@@ -725,8 +735,6 @@ FlipChain::FlipChain(const FlipChainDesc& d) : sites_(d.sites), n_diag_(static_c
   diag_masks_.allocate(std::max(n_diag_, 1) * sizeof(uint64_t));
   diag_coefs_.allocate(std::max(n_diag_, 1) * sizeof(double));
   x_coefs_.allocate(64 * sizeof(double));
-  status_.allocate(sizeof(int));
-  QMBED_CUDA(cudaMemset(status_.get(), 0, sizeof(int)));
   std::vector<double> x(64, 0.0);
   for (int i = 0; i < sites_; ++i) x[i] = d.x_coefs[i];
   if (n_diag_ > 0) {
@@ -818,6 +826,12 @@ void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const 
 namespace qmbed {
 
 namespace {
+
+// QMBED_FLIP_WAIT_POLLS bounds the waits on box copies (tests: 0 gives every copy up at once).
+unsigned wait_polls() {
+  const char* env = std::getenv("QMBED_FLIP_WAIT_POLLS");
+  return env ? static_cast<unsigned>(std::strtoul(env, nullptr, 10)) : kWaitPolls;
+}
 
 template <typename T>
 typename Coef<T>::type host_coef(double c) {
@@ -946,20 +960,11 @@ void FlipChain::apply_boxes(int precision, bool cplx, const void* x, void* out, 
     a.gamma = static_cast<T>(step.gamma);
     a.kr = static_cast<T>(step.kappa_re);
     a.ki = static_cast<T>(step.kappa_im);
-    a.status = status_.as<int>();
+    a.polls = wait_polls();
     launch_box_plan<T, decltype(ctag)::value>(a, plan, step.alpha, host_x_, sites_, stream);
   };
   if (precision == 64) cplx ? run(double{}, std::true_type{}) : run(double{}, std::false_type{});
   else cplx ? run(float{}, std::true_type{}) : run(float{}, std::false_type{});
-}
-
-void FlipChain::check_status() const {
-  int host = 0;
-  QMBED_CUDA(cudaMemcpy(&host, status_.get(), sizeof(int), cudaMemcpyDeviceToHost));
-  if (host != 0) {
-    QMBED_CUDA(cudaMemset(status_.get(), 0, sizeof(int)));
-    raise(QMBED_CUDA_ERROR, "a flip-chain pass timed out waiting for its tile copy");
-  }
 }
 
 }  // namespace qmbed

@@ -54,8 +54,6 @@ class FlipChain {
              cudaStream_t stream) const;
   // Gershgorin-type bounds: |D| max over the diagonal terms plus sum |x|.
   double norm_bound() const;
-  // Raises when a box launch recorded a timed-out wait (and clears it).
-  void check_status() const;
 
  private:
   int sites_;
@@ -77,7 +75,6 @@ class FlipChain {
                    const FlipStep& step, cudaStream_t stream, const BoxPlan& plan) const;
   mutable std::mutex tables_mu_;
   mutable BoxTables box_tables_[4][2];  // [precision, complex][box width]
-  DeviceBuffer status_;
   std::vector<uint64_t> host_diag_masks_;
   std::vector<double> host_diag_coefs_, host_x_;
 };
