@@ -28,9 +28,6 @@ constexpr size_t kGuaranteedDense = 128;
 constexpr size_t kAutomaticDense = 256;
 constexpr size_t kFullKrylovDenseFallback = 2048;
 constexpr size_t kTridiagonalWindow = 96;
-// Lanczos steps queued before the host reads their records: a run that ends
-// early has at most this many steps to throw away.
-constexpr size_t kQueuedSteps = 32;
 constexpr double kEps = 2.220446049250313e-16;
 const double kDgks = 1.0 / std::sqrt(2.0);
 // FP32 vectors resolve residuals to about 1e-7 of the spectral scale; the mixed
@@ -271,82 +268,44 @@ EigshResult lanczos_window(Ctx& c, const EigshOptions& o, const void* initial_de
   }
   std::vector<double> alphas, betas;
   size_t passes = 0, seconds = 0, size = 0;
-  // FP64 steps queue up to kQueuedSteps at a time; the loop below takes over
-  // where a step needs a second pass that the queue does not make, and for FP32.
-  size_t begin = 0;
-  bool finished = false;
-  while (c.prec == 64 && begin < krylov && !finished) {
-    const size_t end = std::min(krylov, begin + kQueuedSteps);
-    c.ops.lanczos_begin(static_cast<int>(end - begin), static_cast<int>(end), begin > 0 ? betas[begin - 1] : 0.0);
-    for (size_t it = begin; it < end; ++it) {
-      c.apply(V.col(static_cast<int>(it)), out);
-      c.ops.lanczos_step(static_cast<const double*>(V.col(0)), n, static_cast<int>(it + 1), static_cast<double*>(out),
-                         it + 1 < krylov ? static_cast<double*>(V.col(static_cast<int>(it + 1))) : nullptr, c.cplx);
-    }
-    std::vector<OrthoRecord> records;
-    c.ops.lanczos_finish(records);
-    const bool whole = c.ops.lanczos_fused(n, static_cast<int>(end));
-    size_t it = begin;
-    for (; it < end && !finished; ++it) {
-      const OrthoRecord& r = records[it - begin];
-      // redone below from this step on: a second pass is due, or the next column was not written (norms that are not finite)
-      if ((r.second && !whole) || (!r.ok && !(r.norm <= 1.0e-14))) break;
-      alphas.push_back(r.h.back().real());
-      size = it + 1;
-      passes += r.second ? 2 : 1;
-      seconds += r.second ? 1 : 0;
-      if (it + 1 == krylov || r.norm <= 1.0e-14) finished = true;
-      else betas.push_back(r.norm);
-    }
-    c.applications -= end - it;
-    begin = it;
-    if (it < end) break;
-  }
-  for (size_t it = begin; it < krylov && !finished; ++it) {
+  if (c.prec == 64)
+    c.ops.lanczos_run(
+        static_cast<double*>(V.col(0)), n, static_cast<int>(krylov), static_cast<double*>(out), c.cplx,
+        [&](int it) { c.op.apply(c.prec, c.cplx, V.col(it), out); },
+        [&](const OrthoRecord& r) {
+          ++c.applications;
+          alphas.push_back(r.h.back().real());
+          ++size;
+          passes += r.second ? 2 : 1;
+          seconds += r.second ? 1 : 0;
+          if (size == krylov || r.norm <= 1.0e-14) return false;
+          betas.push_back(r.norm);
+          return true;
+        });
+  for (size_t it = 0; c.prec != 64 && it < krylov; ++it) {
     c.apply(V.col(static_cast<int>(it)), out);
     const int m = static_cast<int>(it + 1);
     double alpha, before, beta;
-    if (c.prec == 64) {
-      // FP64: alpha, the three-term residual norm and one classical pass over
-      // the whole basis come from two sweeps and one host synchronisation;
-      // dgks_reorthogonalize (src/solve/mod.rs:1050-1099) repeats the pass
-      double before_sq, after_sq;
-      C64 a;
-      c.ops.gram_schmidt_pass(static_cast<const double*>(V.col(0)), n, m, it > 0 ? betas[it - 1] : 0.0, true,
-                              static_cast<double*>(out), c.cplx, &before_sq, &after_sq, &a);
-      alpha = a.real();
-      before = std::sqrt(std::max(before_sq, 0.0));
-      beta = std::sqrt(std::max(after_sq, 0.0));
-      passes += 1;
-      if (before > kEps && beta <= kDgks * before) {
-        c.ops.gram_schmidt_pass(static_cast<const double*>(V.col(0)), n, m, 0.0, false, static_cast<double*>(out),
-                                c.cplx, &before_sq, &after_sq, nullptr);
-        beta = std::sqrt(std::max(after_sq, 0.0));
-        passes += 1;
-        seconds += 1;
-      }
+    C64 a;
+    c.ops.dots(V.col(static_cast<int>(it)), n, 1, out, n, c.prec, c.cplx, &a);
+    alpha = a.real();
+    if (it > 0) {
+      const C64 h[2] = {C64(betas[it - 1], 0.0), C64(alpha, 0.0)};
+      before = c.ops.subtract(V.col(static_cast<int>(it - 1)), n, 2, h, out, n, c.prec, c.cplx, true);
     } else {
-      C64 a;
-      c.ops.dots(V.col(static_cast<int>(it)), n, 1, out, n, c.prec, c.cplx, &a);
-      alpha = a.real();
-      if (it > 0) {
-        const C64 h[2] = {C64(betas[it - 1], 0.0), C64(alpha, 0.0)};
-        before = c.ops.subtract(V.col(static_cast<int>(it - 1)), n, 2, h, out, n, c.prec, c.cplx, true);
-      } else {
-        const C64 h[1] = {C64(alpha, 0.0)};
-        before = c.ops.subtract(V.col(0), n, 1, h, out, n, c.prec, c.cplx, true);
-      }
-      // dgks_reorthogonalize over the whole basis (src/solve/mod.rs:1050-1099)
-      std::vector<C64> h(m);
+      const C64 h[1] = {C64(alpha, 0.0)};
+      before = c.ops.subtract(V.col(0), n, 1, h, out, n, c.prec, c.cplx, true);
+    }
+    // dgks_reorthogonalize over the whole basis (src/solve/mod.rs:1050-1099)
+    std::vector<C64> h(m);
+    c.ops.dots(V.col(0), n, m, out, n, c.prec, c.cplx, h.data());
+    beta = c.ops.subtract(V.col(0), n, m, h.data(), out, n, c.prec, c.cplx, true);
+    passes += 1;
+    if (before > kEps && beta <= kDgks * before) {
       c.ops.dots(V.col(0), n, m, out, n, c.prec, c.cplx, h.data());
       beta = c.ops.subtract(V.col(0), n, m, h.data(), out, n, c.prec, c.cplx, true);
       passes += 1;
-      if (before > kEps && beta <= kDgks * before) {
-        c.ops.dots(V.col(0), n, m, out, n, c.prec, c.cplx, h.data());
-        beta = c.ops.subtract(V.col(0), n, m, h.data(), out, n, c.prec, c.cplx, true);
-        passes += 1;
-        seconds += 1;
-      }
+      seconds += 1;
     }
     alphas.push_back(alpha);
     size = it + 1;

@@ -1674,6 +1674,54 @@ void BlockOps::lanczos_step(const double* A, uint64_t n, int m, double* w, doubl
   QMBED_LAUNCH_CHECK();
 }
 
+// Steps queue up, 8 at first and twice as many each time up to 32, so that a run
+// that ends early throws away no more steps than it has used, or seven. A step
+// that the queue leaves short (a second pass is due, or the norm is below the
+// kernels' 1e-14 or not finite and the next column was not written) is finished
+// here if it is the queue's last, whose vector is still in w; else it is made
+// again as a queue of one. After such a step queues start over from one, so a
+// run of them costs what it would step by step (with queues of 32 throughout,
+// each of them threw away up to 31 products).
+constexpr int kFirstQueue = 8, kLongestQueue = 32;
+
+void BlockOps::lanczos_run(double* A, uint64_t n, int capacity, double* w, bool cplx,
+                           const std::function<void(int)>& product,
+                           const std::function<bool(const OrthoRecord&)>& take) {
+  auto col = [&](int j) { return A + static_cast<uint64_t>(j) * n * (cplx ? 2 : 1); };
+  std::vector<OrthoRecord> records;
+  double beta = 0.0;
+  bool on = true;
+  int queue = kFirstQueue;
+  for (int index = 0; on && index < capacity;) {
+    const int end = std::min(capacity, index + queue);
+    fused_.begin(end - index, end, beta, stream_);
+    for (int i = index; i < end; ++i) {
+      product(i);
+      lanczos_step(A, n, i + 1, w, i + 1 < capacity ? col(i + 1) : nullptr, cplx);
+    }
+    fused_.finish(records, stream_);
+    int i = index;
+    bool stepwise = false;
+    for (; on && i < end; ++i) {
+      OrthoRecord& r = records[static_cast<size_t>(i - index)];
+      const bool second_due = r.second && !fused_.applies(n, i + 1);
+      const bool left_short = second_due || !r.ok;
+      stepwise = stepwise || left_short;
+      if (left_short && i + 1 < end) break;
+      if (second_due) {
+        double unused_sq = 0.0, after_sq = 0.0;
+        gram_schmidt_pass(A, n, i + 1, 0.0, false, w, cplx, &unused_sq, &after_sq, nullptr);
+        r.norm = std::sqrt(std::max(after_sq, 0.0));
+      }
+      on = take(r);
+      beta = r.norm;
+      if (on && left_short && i + 1 < capacity) scale_into(w, col(i + 1), n, beta, 64, cplx);
+    }
+    queue = stepwise ? 1 : std::min(2 * queue, kLongestQueue);
+    index = i;
+  }
+}
+
 void BlockOps::project_out(const double* A, uint64_t n, int m, const double* src, double* w, bool cplx, C64* h,
                            double* src_norm_sq, double* out_norm_sq) {
   if (m <= 0 || n == 0) raise(QMBED_INTERNAL_STATE, "empty projection");

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <complex>
+#include <functional>
 #include <vector>
 
 #include "common.cuh"
@@ -54,17 +55,14 @@ class BlockOps {
   // host synchronisation.
   void project_out(const double* A, uint64_t n, int m, const double* src, double* w, bool cplx, C64* h,
                    double* src_norm_sq, double* out_norm_sq);
-  // Lanczos steps queued without a host round trip, up to `steps` of them on
-  // panels of at most m columns (`beta`: the norm before the first step). A
-  // step orthogonalises w against the m columns of A as gram_schmidt_pass does
-  // (three-term test) and writes w / |w| to `slot` (when given and |w| > 1e-14);
-  // lanczos_finish waits for the records. Vectors that the fused kernel serves
-  // get their DGKS second pass on the device; with larger ones a record whose
-  // `second` is set is short of it, and it and the steps after it are to be redone.
-  bool lanczos_fused(uint64_t n, int m) const { return fused_.applies(n, m); }
-  void lanczos_begin(int steps, int m, double beta) { fused_.begin(steps, m, beta, stream_); }
-  void lanczos_step(const double* A, uint64_t n, int m, double* w, double* slot, bool cplx);
-  void lanczos_finish(std::vector<OrthoRecord>& records) { fused_.finish(records, stream_); }
+  // FP64 Lanczos steps on the panel A (columns of n rows, the first one given,
+  // up to `capacity` of them): `product(i)` queues w = H a_i on the stream, the
+  // step orthogonalises w against a_0 .. a_i as gram_schmidt_pass does (with the
+  // three-term DGKS test and its second pass) and writes w / |w| to a_{i+1}.
+  // `take` gets the steps' records in order and says whether the run goes on.
+  // Steps are queued ahead of the host; it reads their records together.
+  void lanczos_run(double* A, uint64_t n, int capacity, double* w, bool cplx, const std::function<void(int)>& product,
+                   const std::function<bool(const OrthoRecord&)>& take);
   // One vector against m columns with the second pass, into slot (w when null).
   FusedOrtho& fused() { return fused_; }
   double norm(const void* w, uint64_t n, int precision, bool cplx);
@@ -106,6 +104,10 @@ class BlockOps {
   void release_workspace();
 
  private:
+  // One queued step, its record on the device. The fused kernel makes the second
+  // pass itself; the separate launches for larger vectors leave w after the
+  // first, with the record's `second` set.
+  void lanczos_step(const double* A, uint64_t n, int m, double* w, double* slot, bool cplx);
   void ensure_partials(size_t doubles);
   void ensure_coeffs(size_t bytes);
   int device_;

@@ -28,8 +28,6 @@ namespace qmbed {
 namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
-constexpr double kDgks = 0.70710678118654752440;  // 1/sqrt(2)
-constexpr int kQueuedSteps = 32;  // Lanczos steps queued before the host reads their records
 
 int grid_for(uint64_t n, int sms) {
   return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 8ull * sms)));
@@ -116,11 +114,6 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   if (!d.lent && d.basis.bytes() < panel_bytes) d.basis.allocate(panel_bytes);  // kept across repeated runs
   Scratch w(ops, 21, n * width);
   auto col = [&](int j) { return static_cast<char*>(d.panel()) + static_cast<size_t>(j) * n * width; };
-  // one Gram-Schmidt pass over q_0 .. q_{m-1}; returns (|w'|^2, |w''|^2, alpha)
-  auto pass = [&](int m, double beta, bool three_term, double* before_sq, double* after_sq, C64* alpha) {
-    ops.gram_schmidt_pass(static_cast<double*>(d.panel()), n, m, beta, three_term, w.as<double>(), cplx, before_sq, after_sq,
-                          alpha);
-  };
 
   // normalize (src/solve/mod.rs:694-705) on the caller's vector
   d.initial_norm = ops.norm(initial, n, 64, initial_cplx);
@@ -140,68 +133,19 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   d.applications = 0;
   d.second_passes = 0;
   std::vector<double> betas;
-  double previous_beta = 0.0;
-  // Steps queue up to kQueuedSteps at a time (no host round trip between
-  // them); one that needs a second pass the queue does not make, or whose next
-  // column it did not write although the run goes on (norms up to the kernels'
-  // 1e-14 that are above the tolerance), is redone by the loop below, which
-  // then goes on step by step to the next queue.
-  bool finished = false;
-  for (int index = 0; index < capacity && !finished; ++index) {
-    {
-      const int end = std::min(capacity, index + kQueuedSteps);
-      ops.lanczos_begin(end - index, end, previous_beta);
-      for (int i = index; i < end; ++i) {
-        op.apply(64, cplx, col(i), w.get());
-        ops.lanczos_step(static_cast<double*>(d.panel()), n, i + 1, w.as<double>(),
-                         i + 1 < capacity ? reinterpret_cast<double*>(col(i + 1)) : nullptr, cplx);
-      }
-      std::vector<OrthoRecord> records;
-      ops.lanczos_finish(records);
-      const bool whole = ops.lanczos_fused(n, end);
-      int i = index;
-      for (; i < end && !finished; ++i) {
-        const OrthoRecord& r = records[static_cast<size_t>(i - index)];
-        if ((r.second && !whole) || (!r.ok && r.norm > tolerance)) break;
+  ops.lanczos_run(
+      static_cast<double*>(d.panel()), n, capacity, w.as<double>(), cplx,
+      [&](int i) { op.apply(64, cplx, col(i), w.get()); },
+      [&](const OrthoRecord& r) {
         ++d.applications;
-        if (std::fabs(r.h.back().imag()) > std::max(tolerance, 1.0e-10)) raise(QMBED_NON_HERMITIAN, "");
+        // alpha = <q_i, w> is the last overlap of the first pass
+        const C64 alpha = r.h.back();
+        if (std::fabs(alpha.imag()) > std::max(tolerance, 1.0e-10)) raise(QMBED_NON_HERMITIAN, "");
         if (r.second) ++d.second_passes;
-        d.diagonal.push_back(r.h.back().real());
+        d.diagonal.push_back(alpha.real());
         betas.push_back(r.norm);
-        previous_beta = r.norm;
-        finished = i + 1 == capacity || !(r.norm > tolerance);
-      }
-      index = i;
-      if (finished) break;
-      if (i == end) {
-        --index;  // the next queue starts here
-        continue;
-      }
-    }
-    op.apply(64, cplx, col(index), w.get());
-    ++d.applications;
-    // alpha = <q_index, w> is the last overlap of the pass; the pass also
-    // yields the norm of the three-term residual (before reorthogonalisation)
-    double before_sq, after_sq, unused_sq;
-    C64 alpha, again;
-    pass(index + 1, previous_beta, true, &before_sq, &after_sq, &alpha);
-    if (std::fabs(alpha.imag()) > std::max(tolerance, 1.0e-10)) raise(QMBED_NON_HERMITIAN, "");
-    const double before = std::sqrt(std::max(before_sq, 0.0));
-    double beta = std::sqrt(std::max(after_sq, 0.0));
-    if (before > kEps && beta <= kDgks * before) {  // DGKS: repeat the pass once
-      pass(index + 1, 0.0, false, &unused_sq, &after_sq, &again);
-      beta = std::sqrt(std::max(after_sq, 0.0));
-      ++d.second_passes;
-    }
-    d.diagonal.push_back(alpha.real());
-    betas.push_back(beta);
-    if (index + 1 < capacity && beta > tolerance) {
-      ops.scale_into(w.get(), col(index + 1), n, beta, 64, cplx);
-      previous_beta = beta;
-    } else {
-      break;
-    }
-  }
+        return r.norm > tolerance;
+      });
   ops.sync();
   d.size = static_cast<int>(d.diagonal.size());
   d.off_diagonal.assign(betas.begin(), betas.end() - 1);
