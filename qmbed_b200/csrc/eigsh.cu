@@ -382,6 +382,7 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
   W.alloc(n, m, c.prec, c.cplx, c.ops, 13);      // applied actions of the basis
   C.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 14);   // Ritz candidates of this cycle
   CA.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 15);  // their actions
+  if (c.prec == 64 && c.ops.fused().applies(n, k + m)) c.ops.fused().reserve(m, k + m, c.ops.stream());
   const int retain_cap = std::max(keep_cap, n_initial);
   RC.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 16);   // vectors retained for the next cycle
   RCA.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 17);  // their actions

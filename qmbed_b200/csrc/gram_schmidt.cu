@@ -300,13 +300,10 @@ bool FusedOrtho::applies(uint64_t n, int m) const {
   return n > 0 && m >= 1 && m <= kMaxColumns && n <= static_cast<uint64_t>(kMaxRows) * sms_;
 }
 
-void FusedOrtho::begin(int steps, int m, double beta, cudaStream_t stream) {
-  steps_ = steps;
-  cap_ = kRecordHead + 2 * m;
-  count_ = 0;
-  columns_.clear();
-  const size_t bytes = sizeof(GridState) + static_cast<size_t>(steps) * cap_ * sizeof(double);
-  const size_t part = 2 * (static_cast<size_t>(m) * 2 + 2) * sms_ * sizeof(double);
+void FusedOrtho::reserve(int steps, int m, cudaStream_t stream) {
+  const size_t bytes = sizeof(GridState) + static_cast<size_t>(steps) * (kRecordHead + 2 * m) * sizeof(double);
+  // the fused kernel's partial sums; wider panels take other kernels, which have their own
+  const size_t part = 2 * (static_cast<size_t>(std::min(m, kMaxColumns)) * 2 + 2) * sms_ * sizeof(double);
   if (state_.bytes() < bytes || partials_.bytes() < part) {
     QMBED_CUDA(cudaStreamSynchronize(stream));
     if (state_.bytes() < bytes) state_.allocate(bytes);
@@ -318,6 +315,15 @@ void FusedOrtho::begin(int steps, int m, double beta, cudaStream_t stream) {
     QMBED_CUDA(cudaMallocHost(&host_, bytes));
     host_bytes_ = bytes;
   }
+}
+
+void FusedOrtho::begin(int steps, int m, double beta, cudaStream_t stream) {
+  reserve(steps, m, stream);
+  steps_ = steps;
+  cap_ = kRecordHead + 2 * m;
+  count_ = 0;
+  columns_.clear();
+  const size_t bytes = sizeof(GridState) + static_cast<size_t>(steps) * cap_ * sizeof(double);
   GridState head{};
   head.first[1] = beta;
   std::memcpy(host_, &head, sizeof head);

@@ -32,6 +32,9 @@ class FusedOrtho {
 
   // Whether panels of n rows and up to m columns take the fused kernel.
   bool applies(uint64_t n, int m) const;
+  // Buffers for runs of up to `steps` records on panels of up to m columns, so
+  // that none of them allocates.
+  void reserve(int steps, int m, cudaStream_t stream);
   // Starts a run of at most `steps` records for panels of up to `m` columns;
   // `beta` stands for the norm of the record before the first.
   void begin(int steps, int m, double beta, cudaStream_t stream);

@@ -955,6 +955,18 @@ int kept_columns(uint64_t n, bool cplx) {
   return static_cast<int>(std::min<uint64_t>(kKeptPanelBytes / (n * (cplx ? 16 : 8)), 1u << 20));
 }
 
+// Rows of a panel_dot_kernel block: 256..2048, for about eight blocks per SM.
+int panel_slab(uint64_t n, int sms) {
+  const uint64_t target = (n + 8ull * sms - 1) / (8ull * sms);
+  return static_cast<int>(std::min<uint64_t>(kMaxSlab, std::max<uint64_t>(256, (target + 255) / 256 * 256)));
+}
+
+// Doubles of partial sums that the overlaps with m columns take.
+size_t panel_partials(uint64_t n, int m, int sms) {
+  const int slab = panel_slab(n, sms);
+  return static_cast<size_t>(m) * ((n + slab - 1) / slab) * 2 + 2 * static_cast<size_t>(m) + 64;
+}
+
 constexpr int kOrthoThreads = 256;
 constexpr int kOrthoChunk = 8;
 
@@ -1347,11 +1359,9 @@ void BlockOps::dots_device(const void* A, uint64_t ld, int m, const void* w, uin
   if (m <= 0 || n == 0) return;
   int G;
   if (precision == 64) {
-    // slabs of 256..2048 rows, sized for about eight blocks per SM
-    const uint64_t target = (n + 8ull * sms_ - 1) / (8ull * sms_);
-    const int slab = static_cast<int>(std::min<uint64_t>(kMaxSlab, std::max<uint64_t>(256, (target + 255) / 256 * 256)));
+    const int slab = panel_slab(n, sms_);
     G = static_cast<int>((n + slab - 1) / slab);
-    ensure_partials(static_cast<size_t>(m) * G * 2 + 2 * static_cast<size_t>(m) + 64);
+    ensure_partials(panel_partials(n, m, sms_));
     const size_t smem = static_cast<size_t>(slab) * (cplx ? 16 : 8);
     if (cplx)
       launch_dependent(panel_dot_kernel<true>, G, kThreads, smem, stream_, static_cast<const double*>(A), ld, m,
@@ -1688,6 +1698,12 @@ void BlockOps::lanczos_run(double* A, uint64_t n, int capacity, double* w, bool 
                            const std::function<void(int)>& product,
                            const std::function<bool(const OrthoRecord&)>& take) {
   auto col = [&](int j) { return A + static_cast<uint64_t>(j) * n * (cplx ? 2 : 1); };
+  // every step's buffers before the first: an allocation between them waits for the device
+  fused_.reserve(std::min(capacity, kLongestQueue), capacity, stream_);
+  if (!fused_.applies(n, capacity)) {
+    ensure_coeffs(static_cast<size_t>(capacity) * 16);
+    ensure_partials(std::max(panel_partials(n, capacity, sms_), 8 * static_cast<size_t>(sms_) + 64));
+  }
   std::vector<OrthoRecord> records;
   double beta = 0.0;
   bool on = true;
