@@ -10,7 +10,10 @@
 // compaction writes them in rank order, which is ascending numeric order.
 #include <chrono>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <numeric>
+#include <vector>
 
 #include "basis.cuh"
 #include "device_util.cuh"
@@ -21,6 +24,13 @@ void DeviceBuffer::allocate(size_t bytes) {
   release();
   if (bytes == 0) return;
   cudaError_t status = cudaMalloc(&ptr_, bytes);
+  if (status == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    int device = 0;
+    QMBED_CUDA(cudaGetDevice(&device));
+    BlockPool::trim(device);
+    status = cudaMalloc(&ptr_, bytes);
+  }
   if (status != cudaSuccess) {
     ptr_ = nullptr;
     (void)cudaGetLastError();
@@ -34,6 +44,99 @@ void DeviceBuffer::release() {
   if (ptr_) cudaFree(ptr_);
   ptr_ = nullptr;
   bytes_ = 0;
+}
+
+namespace {
+
+struct PooledBlock {
+  void* ptr;
+  size_t bytes;
+};
+struct DevicePool {
+  std::vector<PooledBlock> blocks;  // oldest first
+  size_t bytes = 0;
+  int handles = 0;
+};
+std::mutex g_pool_mu;
+
+std::map<int, DevicePool>& pools() {
+  static auto* all = new std::map<int, DevicePool>;  // never destroyed: handles may outlive static objects
+  return *all;
+}
+
+void free_blocks(const std::vector<PooledBlock>& blocks) {
+  for (const PooledBlock& b : blocks) cudaFree(b.ptr);
+}
+
+std::vector<PooledBlock> take_all(DevicePool& pool) {
+  std::vector<PooledBlock> all;
+  all.swap(pool.blocks);
+  pool.bytes = 0;
+  return all;
+}
+
+}  // namespace
+
+void* BlockPool::take(size_t bytes, size_t* capacity) {
+  int device = 0;
+  QMBED_CUDA(cudaGetDevice(&device));
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  DevicePool& pool = pools()[device];
+  // the smallest block that is no more than a quarter too large
+  auto best = pool.blocks.end();
+  for (auto b = pool.blocks.begin(); b != pool.blocks.end(); ++b)
+    if (b->bytes >= bytes && b->bytes <= bytes + bytes / 4 && (best == pool.blocks.end() || b->bytes < best->bytes))
+      best = b;
+  if (best == pool.blocks.end()) return nullptr;
+  void* block = best->ptr;
+  *capacity = best->bytes;
+  pool.bytes -= best->bytes;
+  pool.blocks.erase(best);
+  return block;
+}
+
+void BlockPool::give(void* block, size_t capacity, int device) {
+  std::vector<PooledBlock> out;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool& pool = pools()[device];
+    if (capacity > kLimit || pool.handles == 0) {
+      out.push_back({block, capacity});
+    } else {
+      while (pool.bytes + capacity > kLimit) {
+        out.push_back(pool.blocks.front());
+        pool.bytes -= pool.blocks.front().bytes;
+        pool.blocks.erase(pool.blocks.begin());
+      }
+      pool.blocks.push_back({block, capacity});
+      pool.bytes += capacity;
+    }
+  }
+  free_blocks(out);
+}
+
+void BlockPool::trim(int device) {
+  std::vector<PooledBlock> out;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    out = take_all(pools()[device]);
+  }
+  free_blocks(out);
+}
+
+void BlockPool::attach(int device) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ++pools()[device].handles;
+}
+
+void BlockPool::detach(int device) {
+  std::vector<PooledBlock> out;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool& pool = pools()[device];
+    if (--pool.handles == 0) out = take_all(pool);
+  }
+  free_blocks(out);
 }
 
 namespace {

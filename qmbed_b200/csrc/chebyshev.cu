@@ -73,7 +73,7 @@ void chebyshev_run(const SpinOperator& op, const double* initial, cudaMemcpyKind
   const uint64_t n = op.dim();
   const size_t es = precision == 64 ? 16 : 8;
   const cudaStream_t s = ops.stream();
-  Scratch staging(ops, 24, n * 16), buf_psi(ops, 25, n * es), buf_a(ops, 26, n * es), buf_b(ops, 27, n * es);
+  Scratch staging(ops, n * 16), buf_psi(ops, n * es), buf_a(ops, n * es), buf_b(ops, n * es);
   void* psi = buf_psi.get();
   void* b1 = buf_a.get();
   void* b2 = buf_b.get();

@@ -86,6 +86,13 @@ class DeviceBuffer {
   }
   void allocate(size_t bytes);
   void release();
+  // The allocation, now the caller's.
+  void* detach() {
+    void* p = ptr_;
+    ptr_ = nullptr;
+    bytes_ = 0;
+    return p;
+  }
   template <typename T>
   T* as() const { return static_cast<T*>(ptr_); }
   void* get() const { return ptr_; }
@@ -94,6 +101,24 @@ class DeviceBuffer {
  private:
   void* ptr_ = nullptr;
   size_t bytes_ = 0;
+};
+
+// Device blocks that finished calls leave for the next ones of the process (the
+// driver takes 0.1 to 5 ms per allocation and free): at most kLimit bytes per
+// device, the oldest freed first. They are given back before an allocation of
+// the library fails, and when the device's last handle with solver buffers is
+// gone. A block in here is idle: give() is called after the work on it has
+// completed. Safe to use from several threads.
+class BlockPool {
+ public:
+  static constexpr size_t kLimit = size_t{1} << 30;
+  // A block of at least `bytes` on the current device, `capacity` its size; null when none fits.
+  static void* take(size_t bytes, size_t* capacity);
+  static void give(void* block, size_t capacity, int device);
+  static void trim(int device);
+  // Handles that use the pool on a device.
+  static void attach(int device);
+  static void detach(int device);
 };
 
 constexpr int kMaxArity = 8;

@@ -51,13 +51,13 @@ struct Panel {
     buf.allocate(std::max<size_t>(1, static_cast<size_t>(n) * cols * es()));
     base = buf.get();
   }
-  // in a workspace slot of the handle
-  void alloc(uint64_t n_, int cols_, int prec_, bool cplx_, BlockOps& ops, int slot) {
+  // the call's work buffer
+  void alloc(uint64_t n_, int cols_, int prec_, bool cplx_, BlockOps& ops) {
     n = n_;
     cols = cols_;
     prec = prec_;
     cplx = cplx_;
-    kept.take(ops, slot, static_cast<size_t>(n) * cols * es());
+    kept.take(ops, static_cast<size_t>(n) * cols * es());
     base = kept.get();
   }
   void* col(int j) const { return static_cast<char*>(base) + static_cast<size_t>(j) * n * es(); }
@@ -254,9 +254,9 @@ EigshResult lanczos_window(Ctx& c, const EigshOptions& o, const void* initial_de
   const size_t krylov = std::min({requested, o.max_iterations, static_cast<size_t>(n)});
   if (krylov <= o.eigenpairs) raise(QMBED_INVALID_OPTIONS, "the effective Krylov dimension must exceed eigenpairs");
   Panel V;
-  V.alloc(n, static_cast<int>(krylov), c.prec, c.cplx, c.ops, 19);
+  V.alloc(n, static_cast<int>(krylov), c.prec, c.cplx, c.ops);
   Panel work;
-  work.alloc(n, 1, c.prec, c.cplx, c.ops, 20);
+  work.alloc(n, 1, c.prec, c.cplx, c.ops);
   void* out = work.col(0);
   if (initial_device) {
     c.copy(initial_device, V.col(0));
@@ -378,15 +378,15 @@ EigshResult thick_restart(Ctx& c, const EigshOptions& o, const Panel* initial, i
   auto keep_for = [&](int active) { return std::max(std::min(std::max(active, wider), m / 2), 1); };
   const int keep_cap = keep_for(k);  // candidates per cycle never exceed this
   Panel Q, W, C, CA, RC, RCA, work;
-  Q.alloc(n, k + m, c.prec, c.cplx, c.ops, 12);  // [locked | basis]
-  W.alloc(n, m, c.prec, c.cplx, c.ops, 13);      // applied actions of the basis
-  C.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 14);   // Ritz candidates of this cycle
-  CA.alloc(n, keep_cap, c.prec, c.cplx, c.ops, 15);  // their actions
+  Q.alloc(n, k + m, c.prec, c.cplx, c.ops);  // [locked | basis]
+  W.alloc(n, m, c.prec, c.cplx, c.ops);      // applied actions of the basis
+  C.alloc(n, keep_cap, c.prec, c.cplx, c.ops);   // Ritz candidates of this cycle
+  CA.alloc(n, keep_cap, c.prec, c.cplx, c.ops);  // their actions
   if (c.prec == 64 && c.ops.fused().applies(n, k + m)) c.ops.fused().reserve(m, k + m, c.ops.stream());
   const int retain_cap = std::max(keep_cap, n_initial);
-  RC.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 16);   // vectors retained for the next cycle
-  RCA.alloc(n, retain_cap, c.prec, c.cplx, c.ops, 17);  // their actions
-  work.alloc(n, 1, c.prec, c.cplx, c.ops, 18);
+  RC.alloc(n, retain_cap, c.prec, c.cplx, c.ops);   // vectors retained for the next cycle
+  RCA.alloc(n, retain_cap, c.prec, c.cplx, c.ops);  // their actions
+  work.alloc(n, 1, c.prec, c.cplx, c.ops);
   void* tmp = work.col(0);
   std::vector<double> locked_values, locked_residuals;
   int l = 0;

@@ -95,9 +95,9 @@ class KrylovExp {
  public:
   KrylovExp(const LinearOperatorView& op, BlockOps& ops, size_t krylov)
       : op_(op), ops_(ops), n_(op.dim), m_(static_cast<int>(std::max<uint64_t>(std::min<uint64_t>(krylov, op.dim), 1))) {
-    panel_.take(ops, 32, static_cast<size_t>(m_) * n_ * 16);
-    w_.take(ops, 33, n_ * 16);
-    coeff_.take(ops, 34, static_cast<size_t>(2 * m_) * sizeof(double));
+    panel_.take(ops, static_cast<size_t>(m_) * n_ * 16);
+    w_.take(ops, n_ * 16);
+    coeff_.take(ops, static_cast<size_t>(2 * m_) * sizeof(double));
   }
 
   // lanczos_projection(_real) (src/solve/mod.rs:2909-3054) of a device state
@@ -220,7 +220,7 @@ void evolve(const LinearOperatorView& op, const double* initial, const Evolution
   const uint64_t n = op.dim;
   const cudaStream_t s = ops.stream();
   KrylovExp krylov(op, ops, o.krylov_dimension);
-  Scratch a(ops, 35, n * 16), b(ops, 36, n * 16);
+  Scratch a(ops, n * 16), b(ops, n * 16);
   double* current = a.as<double>();
   double* candidate = b.as<double>();
   QMBED_CUDA(cudaMemcpyAsync(current, initial, n * 16, cudaMemcpyHostToDevice, s));

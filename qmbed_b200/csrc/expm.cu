@@ -146,7 +146,7 @@ size_t expm_apply(const ExpmPlan& plan, const LinearOperatorView& op, void* stat
   cudaStream_t stream = ops.stream();
   const int grid = static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + kThreads - 1) / kThreads,
                                                                              4ULL * ops.sms())));
-  Scratch partials(ops, 28, 2 * grid * sizeof(double));
+  Scratch partials(ops, 2 * grid * sizeof(double));
   std::vector<double> host(2 * grid);
   auto read_max = [&](int stride_, int offset) {
     QMBED_CUDA(cudaMemcpyAsync(host.data(), partials.get(), 2 * grid * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -167,7 +167,7 @@ size_t expm_apply(const ExpmPlan& plan, const LinearOperatorView& op, void* stat
   const C64 eta = std::exp(factor * plan.shift);
   if (!std::isfinite(eta.real()) || !std::isfinite(eta.imag()))
     raise(QMBED_UNSUPPORTED_BACKEND, "exponential action overflowed its scalar trace shift");
-  Scratch term_buf(ops, 29, bytes), applied_buf(ops, 30, bytes), sum(ops, 31, bytes);
+  Scratch term_buf(ops, bytes), applied_buf(ops, bytes), sum(ops, bytes);
   void* term = term_buf.get();
   void* applied = applied_buf.get();
   size_t applications = 0;

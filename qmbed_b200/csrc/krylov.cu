@@ -1272,10 +1272,32 @@ double device_max_shifted_column(const double* diag, const double* offsum, uint6
 BlockOps::BlockOps(int device, cudaStream_t stream)
     : device_(device), stream_(stream), sms_(sm_count(device)), fused_(device, sms_) {
   QMBED_CUDA(cudaSetDevice(device_));
+  BlockPool::attach(device_);
 }
 
 BlockOps::~BlockOps() {
   if (host_results_) cudaFreeHost(host_results_);
+  BlockPool::detach(device_);
+}
+
+void Scratch::take(BlockOps& ops, size_t bytes) {
+  release();
+  QMBED_CUDA(cudaSetDevice(ops.device()));
+  device_ = ops.device();
+  stream_ = ops.stream();
+  bytes = bytes > 0 ? bytes : 1;
+  ptr_ = BlockPool::take(bytes, &bytes_);
+  if (ptr_) return;
+  DeviceBuffer fresh(bytes);
+  bytes_ = bytes;
+  ptr_ = fresh.detach();
+}
+
+void Scratch::release() {
+  if (!ptr_) return;
+  cudaStreamSynchronize(stream_);
+  BlockPool::give(ptr_, bytes_, device_);
+  ptr_ = nullptr;
 }
 
 void* BlockOps::workspace(int slot, size_t bytes) {

@@ -34,6 +34,7 @@ class BlockOps {
 
   cudaStream_t stream() const { return stream_; }
   int sms() const { return sms_; }
+  int device() const { return device_; }
 
   // out[j] = <A_j, w> (conjugate-linear in A) for j < m; with self_sq, also
   // ||w||^2 from the same pass over w.
@@ -121,26 +122,18 @@ class BlockOps {
   size_t host_results_doubles_ = 0;
 };
 
-// Work buffer of one call: a workspace slot of the handle while it is at most
-// kKeptBytes (kept for the next call on the handle and freed with it; the
-// driver takes 0.1 to 5 ms per allocation and free), else an allocation of the
-// call's own. Slots: 0-9 filtered solver, 10 projected eigenproblems, 12-18
-// thick restart, 19-20 Lanczos window, 21-23 thermal Lanczos, 24-27 Chebyshev
-// propagator, 28-31 Taylor action, 32-36 Krylov evolution.
+// Work buffer of one call on a handle's stream: a block of the pool where one
+// fits, else an allocation of its own, and given to the pool at the end. The
+// stream is waited for first: calls that end normally have done so already.
 class Scratch {
  public:
-  static constexpr size_t kKeptBytes = 1ull << 30;
   Scratch() = default;
-  Scratch(BlockOps& ops, int slot, size_t bytes) { take(ops, slot, bytes); }
-  void take(BlockOps& ops, int slot, size_t bytes) {
-    bytes = bytes > 0 ? bytes : 1;
-    if (bytes <= kKeptBytes) {
-      ptr_ = ops.workspace(slot, bytes);
-    } else {
-      own_.allocate(bytes);
-      ptr_ = own_.get();
-    }
-  }
+  Scratch(BlockOps& ops, size_t bytes) { take(ops, bytes); }
+  ~Scratch() { release(); }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  void take(BlockOps& ops, size_t bytes);
+  void release();
   void* get() const { return ptr_; }
   template <typename T>
   T* as() const {
@@ -148,8 +141,10 @@ class Scratch {
   }
 
  private:
-  DeviceBuffer own_;
   void* ptr_ = nullptr;
+  size_t bytes_ = 0;
+  int device_ = 0;
+  cudaStream_t stream_ = nullptr;
 };
 
 // Symmetric tridiagonal eigenproblem on the host by implicit QL with

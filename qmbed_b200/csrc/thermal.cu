@@ -112,7 +112,7 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   const int capacity = static_cast<int>(wanted);
   const size_t panel_bytes = static_cast<size_t>(capacity) * n * width;
   if (!d.lent && d.basis.bytes() < panel_bytes) d.basis.allocate(panel_bytes);  // kept across repeated runs
-  Scratch w(ops, 21, n * width);
+  Scratch w(ops, n * width);
   auto col = [&](int j) { return static_cast<char*>(d.panel()) + static_cast<size_t>(j) * n * width; };
 
   // normalize (src/solve/mod.rs:694-705) on the caller's vector
@@ -378,12 +378,12 @@ void ftlm_sample(const LinearOperatorView& op, int vectors, uint64_t seed, size_
   if (!ok) raise(QMBED_INVALID_OPTIONS, "inverse temperatures must be nonempty, finite, and nonnegative");
   const uint64_t n = op.dim;
   const bool cplx = !op.real;
-  Scratch start(ops, 22, n * (cplx ? 16 : 8));
+  Scratch start(ops, n * (cplx ? 16 : 8));
   log_partition.clear();
   mean_energy.clear();
   lengths.clear();
   LanczosDecomposition d;
-  const Scratch basis(ops, 23, std::min<uint64_t>(std::min<uint64_t>(krylov, n), 8192) * n * (cplx ? 16 : 8));
+  const Scratch basis(ops, std::min<uint64_t>(std::min<uint64_t>(krylov, n), 8192) * n * (cplx ? 16 : 8));
   d.lent = basis.get();
   for (int r = 0; r < vectors; ++r) {
     ftlm_start_vector(op, seed, r, start.as<double>(), ops);
