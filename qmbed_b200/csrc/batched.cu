@@ -709,6 +709,7 @@ ScanResult scan_lowest(const std::vector<std::vector<const SpinOperator*>>& comp
   for (int k = 0; k < K; ++k)
     for (int p = 0; p < P; ++p) coef[static_cast<size_t>(k) * P + p] = coefficients[static_cast<size_t>(std::min(p, points - 1)) * K + k];
   std::vector<SectorDesc> desc(ns);
+  std::vector<std::shared_ptr<const void>> owners;  // of rows assembled for this scan
   uint64_t rows = 0, items = 0;
   size_t set_bytes = 0;  // one vector set (every sector's rows x P complex FP64)
   for (int s = 0; s < ns; ++s) {
@@ -730,6 +731,7 @@ ScanResult scan_lowest(const std::vector<std::vector<const SpinOperator*>>& comp
         raise(QMBED_DIMENSION_MISMATCH, "the components of a sector must share its basis");
       const SpinOperator::ExplicitRows er = op->explicit_rows();
       d.comp[k] = CompRows{er.row_ptr, er.cols, er.values, er.diag, er.row_ptr64 ? 1 : 0, er.diag_complex ? 1 : 0};
+      if (er.owner) owners.push_back(er.owner);
     }
   }
   const int cols = ns * P;

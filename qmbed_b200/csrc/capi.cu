@@ -2065,6 +2065,11 @@ int qmbed_gpu_operator_apply_host(qmbed_operator op, int complex_vectors, const 
 int qmbed_gpu_operator_export_csr(qmbed_operator op, uint64_t* nnz_total, uint64_t* row_ptr, uint32_t* cols,
                                   double* values) {
   return guarded([&] {
+    if (!row_ptr && !cols && !values) {
+      const uint64_t count = op->op->export_count();
+      if (nnz_total) *nnz_total = count;
+      return;
+    }
     std::vector<uint64_t> rp;
     std::vector<uint32_t> c;
     std::vector<C64> v;

@@ -1133,12 +1133,18 @@ SpinOperator::SpinOperator(const SpinOperator& other, RowListTag)
   assemble_row_lists();
 }
 
-const SpinOperator& SpinOperator::row_lists() const {
-  if (!tile_) return *this;
+// The rows of a tiled operator as row lists, for as long as a caller holds them
+// (an export, a scan): kept beside the tiles they would take several times the
+// tiles' memory.
+std::shared_ptr<const SpinOperator> SpinOperator::row_lists() const {
   std::lock_guard<std::mutex> lock(row_lists_mu_);
-  QMBED_CUDA(cudaSetDevice(basis_->device()));
-  if (!row_lists_) row_lists_.reset(new SpinOperator(*this, RowListTag{}));
-  return *row_lists_;
+  std::shared_ptr<const SpinOperator> rows = row_lists_.lock();
+  if (!rows) {
+    QMBED_CUDA(cudaSetDevice(basis_->device()));
+    rows.reset(new SpinOperator(*this, RowListTag{}));
+    row_lists_ = rows;
+  }
+  return rows;
 }
 
 // Rows in tiles of 32 where the operator has that form (one expansion, no
@@ -1506,7 +1512,12 @@ void SpinOperator::apply_with_scratch(int precision, bool complex_vectors, const
 
 SpinOperator::ExplicitRows SpinOperator::explicit_rows() const {
   if (storage_ != kStorageWide) raise(QMBED_UNSUPPORTED_BACKEND, "the operator does not hold rows with explicit values");
-  if (tile_) return row_lists().explicit_rows();
+  if (tile_) {
+    std::shared_ptr<const SpinOperator> rows = row_lists();
+    ExplicitRows r = rows->explicit_rows();
+    r.owner = std::move(rows);
+    return r;
+  }
   ExplicitRows r;
   r.n = dim();
   r.row_ptr64 = row_ptr64_;
@@ -1696,12 +1707,24 @@ void SpinOperator::apply_shift(const SpinBasis& target, const double* x, double*
   QMBED_LAUNCH_CHECK();
 }
 
+uint64_t SpinOperator::export_count() const {
+  QMBED_CUDA(cudaSetDevice(basis_->device()));
+  if (storage_ == kStorageMatrixFree) raise(QMBED_UNSUPPORTED_BACKEND, "matrix-free operators hold no stored rows");
+  const int width = real_ ? 1 : 2;
+  std::vector<double> diag(dim() * width);
+  QMBED_CUDA(cudaMemcpy(diag.data(), (tile_ ? tile_->diag64 : diag64_).get(), diag.size() * 8, cudaMemcpyDeviceToHost));
+  uint64_t count = nnz_off_;
+  for (uint64_t r = 0; r < dim(); ++r)
+    count += diag[width * r] != 0.0 || (width == 2 && diag[2 * r + 1] != 0.0) ? 1 : 0;
+  return count;
+}
+
 void SpinOperator::export_csr(std::vector<uint64_t>& row_ptr, std::vector<uint32_t>& cols,
                               std::vector<C64>& values) const {
   QMBED_CUDA(cudaSetDevice(basis_->device()));
   if (storage_ == kStorageMatrixFree) raise(QMBED_UNSUPPORTED_BACKEND, "matrix-free operators hold no stored rows");
   if (tile_) {
-    row_lists().export_csr(row_ptr, cols, values);
+    row_lists()->export_csr(row_ptr, cols, values);
     return;
   }
   const uint64_t n = dim();

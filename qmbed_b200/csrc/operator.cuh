@@ -118,6 +118,7 @@ class SpinOperator {
     const double* values = nullptr;  // interleaved complex FP64, one per entry
     const double* diag = nullptr;    // FP64: real (n) for real operators, interleaved complex (2n) otherwise
     bool diag_complex = false;
+    std::shared_ptr<const void> owner;  // of the rows where they are assembled for this caller
   };
   ExplicitRows explicit_rows() const;
 
@@ -130,6 +131,8 @@ class SpinOperator {
   bool check_hermitian() const;
 
   // Assembled rows on the host (for tests): row pointer, columns, values.
+  // Entries that export_csr() returns.
+  uint64_t export_count() const;
   void export_csr(std::vector<uint64_t>& row_ptr, std::vector<uint32_t>& cols, std::vector<C64>& values) const;
   // apply_sector_shift (src/operator/mod.rs:2305-2351): these terms applied to
   // a vector of this operator's basis (the source) and reduced into `target`
@@ -162,7 +165,7 @@ class SpinOperator {
   struct RowListTag {};
   // The same operator with its rows as row lists, whatever its own storage.
   SpinOperator(const SpinOperator& other, RowListTag);
-  const SpinOperator& row_lists() const;
+  std::shared_ptr<const SpinOperator> row_lists() const;
 
   void build_instances(const std::vector<TermDesc>& terms, const OperatorChecks& checks);
   void assemble();
@@ -186,7 +189,7 @@ class SpinOperator {
   // Assembled storage: rows in tiles when the operator has that form, else row
   // lists (columns with value codes, or with explicit values).
   std::unique_ptr<TileRows> tile_;
-  mutable std::unique_ptr<SpinOperator> row_lists_;  // of a tiled operator, on first use
+  mutable std::weak_ptr<const SpinOperator> row_lists_;  // of a tiled operator, while a caller holds them
   mutable std::mutex row_lists_mu_;
   std::unique_ptr<FlipProgram> host_prog_;  // until the rows are assembled
   bool hermitian_terms_ = false;            // Hermitian by its products alone
