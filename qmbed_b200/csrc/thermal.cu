@@ -28,6 +28,7 @@ namespace qmbed {
 namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
+constexpr uint64_t kMaxKrylov = 8192;  // the overlaps of one step sit in shared memory (16 bytes each)
 
 int grid_for(uint64_t n, int sms) {
   return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 8ull * sms)));
@@ -107,8 +108,7 @@ void lanczos_ritz_device(const LinearOperatorView& op, const double* initial, bo
   const bool cplx = !d.real;
   const size_t width = cplx ? 16 : 8;
   const uint64_t wanted = std::min<uint64_t>(krylov, n);
-  // the overlaps of one step sit in shared memory (16 bytes each)
-  if (wanted > 8192) raise(QMBED_UNSUPPORTED_BACKEND, "Krylov dimensions above 8192 are not supported");
+  if (wanted > kMaxKrylov) raise(QMBED_UNSUPPORTED_BACKEND, "Krylov dimensions above 8192 are not supported");
   const int capacity = static_cast<int>(wanted);
   const size_t panel_bytes = static_cast<size_t>(capacity) * n * width;
   if (!d.lent && d.basis.bytes() < panel_bytes) d.basis.allocate(panel_bytes);  // kept across repeated runs
@@ -383,8 +383,13 @@ void ftlm_sample(const LinearOperatorView& op, int vectors, uint64_t seed, size_
   mean_energy.clear();
   lengths.clear();
   LanczosDecomposition d;
-  const Scratch basis(ops, std::min<uint64_t>(std::min<uint64_t>(krylov, n), 8192) * n * (cplx ? 16 : 8));
-  d.lent = basis.get();
+  // one panel for all runs (dimensions that lanczos_ritz_device refuses take none)
+  const uint64_t wanted = std::min<uint64_t>(krylov, n);
+  Scratch basis;
+  if (vectors > 0 && wanted <= kMaxKrylov) {
+    basis.take(ops, wanted * n * (cplx ? 16 : 8));
+    d.lent = basis.get();
+  }
   for (int r = 0; r < vectors; ++r) {
     ftlm_start_vector(op, seed, r, start.as<double>(), ops);
     lanczos_ritz_device(op, start.as<double>(), cplx, krylov, tolerance, d, ops, false);
