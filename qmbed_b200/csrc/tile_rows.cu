@@ -315,7 +315,12 @@ __global__ void __launch_bounds__(kFillThreads) tile_fill_kernel(const __grid_co
         continue;
       }
       const double ratio = symmetric ? a.inv_sqrt[257 + a.orbits[r]] * a.inv_sqrt[a.orbits[c]] : 1.0;
-      if (!(hypot(sum.x, sum.y) * ratio > kEps)) continue;
+      if (!(hypot(sum.x, sum.y) * ratio > kEps)) {
+        // entries that cancel are none: the row does not read the column (which may hold an infinity)
+        for (uint32_t j = i; j < kept; ++j)
+          if ((stage[j * 32] & col_mask) == c) a.entries[(static_cast<uint64_t>(base) + j) * 32 + lane] = kNoEntry;
+        continue;
+      }
       ++counted;
       if (a.cplx) continue;
       const unsigned long long bits =
