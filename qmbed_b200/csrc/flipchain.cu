@@ -763,7 +763,7 @@ void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const 
     auto aligned = [](const void* ptr) { return ptr == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
     if (plan.vb > 0 && aligned(x) && aligned(out) && aligned(p) && aligned(q)) {
       const bool over = x == out || (q && q == out);
-      if (over && dim() * static_cast<uint64_t>(esize) >= (256ull << 20))
+      if (over && (!plan.groups.empty() || dim() * static_cast<uint64_t>(esize) >= (256ull << 20)))
         raise(QMBED_INVALID_OPTIONS, "the flip-chain action cannot write over x or q");
       if (!over) {
         apply_boxes(precision, cplx, x, out, p, q, step, stream, plan);
