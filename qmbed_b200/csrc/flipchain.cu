@@ -735,6 +735,9 @@ FlipChain::FlipChain(const FlipChainDesc& d) : sites_(d.sites), n_diag_(static_c
   diag_masks_.allocate(std::max(n_diag_, 1) * sizeof(uint64_t));
   diag_coefs_.allocate(std::max(n_diag_, 1) * sizeof(double));
   x_coefs_.allocate(64 * sizeof(double));
+  // low-bit diagonal tables of the tile kernel (2^tb values of the working
+  // precision, at most kTileBytes each): FP64 table first, FP32 table second
+  tables_.allocate(2 * static_cast<size_t>(kTileBytes));
   std::vector<double> x(64, 0.0);
   for (int i = 0; i < sites_; ++i) x[i] = d.x_coefs[i];
   if (n_diag_ > 0) {
@@ -757,6 +760,7 @@ double FlipChain::norm_bound() const {
 void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
                       const FlipStep& step, cudaStream_t stream) const {
   const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1);
+  prepare_tables(stream);
   {
     const int vbits = log2_int(16 / esize);
     const BoxPlan plan = box_plan(sites_, vbits, dim() * static_cast<uint64_t>(esize), p || q);
@@ -777,14 +781,6 @@ void FlipChain::apply(int precision, bool cplx, const void* x, void* out, const 
   int device = 0, sms = 148;
   QMBED_CUDA(cudaGetDevice(&device));
   QMBED_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  // low-bit diagonal tables (2^tb values of the working precision, at most
-  // kTileBytes each): FP64 table first, FP32 table second
-  const size_t need = 2 * static_cast<size_t>(kTileBytes);
-  if (tables_bytes_ < need) {
-    tables_.allocate(need);
-    tables_bytes_ = need;
-    tables_ready_ = 0;
-  }
   const int table_slot = precision == 64 ? 1 : 2;
   void* table = static_cast<unsigned char*>(tables_.get()) + (precision == 64 ? 0 : kTileBytes);
   if (!(tables_ready_ & table_slot) || table_tb_[table_slot - 1] != tb) {
@@ -881,13 +877,29 @@ void launch_box_plan(BoxArgs<T> base, const BoxPlan& plan, double alpha, const s
 
 }  // namespace
 
-// The diagonal's tables for boxes of 2^vb words, built once per (precision,
-// real or complex); complete before any stream can use them.
-const FlipChain::BoxTables& FlipChain::box_tables(int precision, bool cplx, int vb, cudaStream_t stream) const {
-  const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1), vbits = log2_int(16 / esize);
+// The diagonal's tables for boxes of 2^vb words with vbits state bits inside a
+// word; complete before any stream can use them.
+const FlipChain::BoxTables& FlipChain::box_tables(int vbits, int vb, cudaStream_t stream) const {
   std::lock_guard<std::mutex> lock(tables_mu_);
-  BoxTables& t = box_tables_[(precision == 64 ? 0 : 2) + (cplx ? 1 : 0)][vb == 10 ? 1 : 0];
-  if (t.ready) return t;
+  BoxTables& t = box_tables_[vbits][vb == 10 ? 1 : 0];
+  if (!t.ready) build_box_tables(vbits, vb, stream, t);
+  return t;
+}
+
+// The tables of every element size, on the first call: a later one may be under
+// capture, where nothing can be allocated.
+void FlipChain::prepare_tables(cudaStream_t stream) const {
+  std::lock_guard<std::mutex> lock(tables_mu_);
+  if (tables_prepared_) return;
+  for (int vbits = 0; vbits < 3; ++vbits) {
+    const int vb = box_plan(sites_, vbits, 0, false).vb;
+    BoxTables& t = box_tables_[vbits][vb == 10 ? 1 : 0];
+    if (vb > 0 && !t.ready) build_box_tables(vbits, vb, stream, t);
+  }
+  tables_prepared_ = true;
+}
+
+void FlipChain::build_box_tables(int vbits, int vb, cudaStream_t stream, BoxTables& t) const {
   const uint64_t lanes = (1ull << (kBoxLaneBits + vbits)) - 1, in_box = (1ull << (vb + vbits)) - 1;
   const uint64_t words = in_box & ~lanes;
   const int n_lanes = 1 << (kBoxLaneBits + vbits), n_words = 1 << (vb - kBoxLaneBits);
@@ -934,12 +946,12 @@ const FlipChain::BoxTables& FlipChain::box_tables(int precision, bool cplx, int 
   QMBED_LAUNCH_CHECK();
   QMBED_CUDA(cudaStreamSynchronize(stream));
   t.ready = true;
-  return t;
 }
 
 void FlipChain::apply_boxes(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
                             const FlipStep& step, cudaStream_t stream, const BoxPlan& plan) const {
-  const BoxTables& t = box_tables(precision, cplx, plan.vb, stream);
+  const int esize = (precision == 64 ? 8 : 4) * (cplx ? 2 : 1);
+  const BoxTables& t = box_tables(log2_int(16 / esize), plan.vb, stream);
   unsigned char* base = t.buf.as<unsigned char>();
   auto run = [&](auto ttag, auto ctag) {
     using T = decltype(ttag);

@@ -60,7 +60,6 @@ class FlipChain {
   int n_diag_;
   DeviceBuffer diag_masks_, diag_coefs_, x_coefs_;
   mutable DeviceBuffer tables_;  // low-bit diagonal tables (FP64, FP32)
-  mutable size_t tables_bytes_ = 0;
   mutable int tables_ready_ = 0;  // bit 1: FP64 table, bit 2: FP32 table
   mutable int table_tb_[2] = {0, 0};
   // Box action and the diagonal's tables per box width.
@@ -70,11 +69,14 @@ class FlipChain {
     size_t at_coefs = 0, at_table = 0, at_words = 0, at_high = 0;
     int n_lane = 0, n_word = 0;
   };
-  const BoxTables& box_tables(int precision, bool cplx, int vb, cudaStream_t stream) const;
+  const BoxTables& box_tables(int vbits, int vb, cudaStream_t stream) const;
+  void prepare_tables(cudaStream_t stream) const;
+  void build_box_tables(int vbits, int vb, cudaStream_t stream, BoxTables& t) const;
   void apply_boxes(int precision, bool cplx, const void* x, void* out, const void* p, const void* q,
                    const FlipStep& step, cudaStream_t stream, const BoxPlan& plan) const;
   mutable std::mutex tables_mu_;
-  mutable BoxTables box_tables_[4][2];  // [precision, complex][box width]
+  mutable bool tables_prepared_ = false;
+  mutable BoxTables box_tables_[3][2];  // [state bits inside a word][box width]
   std::vector<uint64_t> host_diag_masks_;
   std::vector<double> host_diag_coefs_, host_x_;
 };
