@@ -739,6 +739,9 @@ struct JacobiElem<true> {
 
 __device__ __forceinline__ double jacobi_sq(double v) { return v * v; }
 __device__ __forceinline__ double jacobi_sq(double2 v) { return v.x * v.x + v.y * v.y; }
+// |v| to the last bits whatever its size: b / |b| is the phase of a unitary rotation
+__device__ __forceinline__ double jacobi_abs(double v) { return fabs(v); }
+__device__ __forceinline__ double jacobi_abs(double2 v) { return hypot(v.x, v.y); }
 // x c - y s f and x s conj(f) + y c: the two rows (or, with f conjugated,
 // columns) of a rotated pair; real data has the phase's sign inside s.
 __device__ __forceinline__ void jacobi_rotate(double& x, double& y, double c, double s, double, double) {
@@ -812,7 +815,7 @@ __global__ void __launch_bounds__(kJacobiMaxThreads)
       q = swap;
     }
     const E b = A[p * ld + q];
-    const double mag = CPLX ? sqrt(jacobi_sq(b)) : fabs(jacobi_re(b));
+    const double mag = jacobi_abs(b);
     double c = 1.0, s = 0.0, fr = 1.0, fi = 0.0;
     if (mag != 0.0) {
       // cos 2 theta = |d| / sqrt(d^2 + 4 |b|^2), d = a_qq - a_pp: c^2 = (1 + cos 2 theta) / 2
