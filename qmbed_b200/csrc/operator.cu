@@ -1350,15 +1350,18 @@ void SpinOperator::apply(int precision, bool complex_vectors, const void* x, voi
   }
   // Stored rows.
   if (tile_) {
-    // symmetry sectors take y over x, as with row lists (whose input is scaled into a buffer of its own)
+    // symmetry sectors take y over x, as with row lists (whose input is scaled into a
+    // buffer of its own); the copy's memory is the stream's, so this may be captured
     const size_t bytes = vector_bytes(precision, cplx);
-    const void* from = x;
     if (basis_->symmetric() && overlap(x, y, bytes)) {
-      ensure_scratch(precision, cplx);
-      QMBED_CUDA(cudaMemcpyAsync(scaled_x_.get(), x, bytes, cudaMemcpyDeviceToDevice, stream));
-      from = scaled_x_.get();
+      void* copy = nullptr;
+      QMBED_CUDA(cudaMallocAsync(&copy, bytes, stream));
+      QMBED_CUDA(cudaMemcpyAsync(copy, x, bytes, cudaMemcpyDeviceToDevice, stream));
+      tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, copy, y, stream);
+      QMBED_CUDA(cudaFreeAsync(copy, stream));
+      return;
     }
-    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, from, y, stream);
+    tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, x, y, stream);
     return;
   }
   const bool scaled = basis_->symmetric();

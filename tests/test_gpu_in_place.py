@@ -1,8 +1,8 @@
 """H.v of symmetry sectors with stored rows, the output over the input.
 
 Such a call gives the bytes of the call with two vectors: the rows read a copy
-of the input (the regular entry keeps one buffer of its own for it, the
-allocation-free entry its fixed array). Sectors of one tile, of a few, of the
+of the input (in the stream's own memory, or in the allocation-free entry's
+fixed array). Sectors of one tile, of a few, of the
 four-warp and the one-warp split, real, complex rows and complex vectors.
 """
 
@@ -25,4 +25,25 @@ def test_output_over_the_input(sites, momentum, parity, precision, entry):
         want = torch.full_like(x, float("nan"))
         getattr(op, entry)(x, want, precision=precision, complex_vectors=cplx)
         getattr(op, entry)(x, x, precision=precision, complex_vectors=cplx)
+        assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("entry", ["apply_device", "apply_device_noalloc"])
+def test_output_over_the_input_under_capture(entry):
+    """After calls with two vectors only: the first call of the other kind may be a captured one."""
+    import torch
+    from qmbed_b200 import GpuBasis, GpuOperator, heisenberg_terms
+    op = GpuOperator(GpuBasis(20, up=10, momentum=0, parity=1), heisenberg_terms(20, delta=0.4))
+    start = torch.randn(op.dim, device="cuda", dtype=torch.float64)
+    once, twice = torch.empty_like(start), torch.empty_like(start)
+    getattr(op, entry)(start, once)
+    getattr(op, entry)(once, twice)
+    x = start.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        getattr(op, entry)(x, x, stream=torch.cuda.current_stream().cuda_stream)
+    for want in (once, twice):
+        graph.replay()
+        torch.cuda.synchronize()
         assert torch.equal(x, want)
