@@ -63,6 +63,9 @@ def test_an_allocation_that_needs_the_pool():
     _thermal(op)  # leaves its panel of 575 MB in the pool
     other = GpuBasis(28, up=14, momentum=3)
     filler = torch.empty(_free() - (200 << 20), device="cuda", dtype=torch.uint8)
-    rows = GpuOperator(other, heisenberg_terms(28))  # 1.4 million complex rows: 230 MB
-    del filler
+    try:
+        rows = GpuOperator(other, heisenberg_terms(28))  # 1.4 million complex rows: 230 MB
+    finally:
+        del filler
+        torch.cuda.empty_cache()  # the other tests' memory
     assert rows.info()["nnz_offdiag"] > 0 and op.dim > 0
