@@ -1283,8 +1283,9 @@ __device__ __forceinline__ uint32_t rank32(uint64_t t, const uint32_t* tab, int 
 // shared memory (index_transition, src/basis/mod.rs:1561-1580). HOLES: the
 // table has states outside the sector. CC: complex characters; CV: complex vectors.
 //
-// Bound by the latency of the two dependent scattered reads (table, vector) at
-// 82% of the warp slots, with integer issue at 53%. The kernels it stands in
+// Bound by the latency of the two dependent scattered reads (table, vector):
+// Heisenberg of 28 sites in FP32 has 62% of the warp slots active, 48% of the
+// issue slots used and no unit above half of its rate. The kernels it stands in
 // for popped the active bonds of every lane (hop_tile_kernel: 104 instructions
 // per transition, ALU pipe 67%; hv_tile_kernel about 230, with the rank of a
 // two-site exchange rebuilt from chunk tables). Measured: Heisenberg of 28

@@ -953,6 +953,10 @@ int stream_grid(uint64_t n, int sms) {
 // sweep over a panel beyond the L2 drives out the columns it is about to need
 // otherwise). Two Lanczos runs of 100 steps at 718,146 rows (28 sites): 26.5 ms
 // without, 25.4 at 30 MB, 25.3 at 40 to 50, 25.5 at 70, 26.6 with none kept.
+// Other sizes, none / 24 / 48 / 96 MB: 200,474 rows, 100 steps 9.7 / 9.6 / 9.6 / 9.9
+// ms; 400,023 complex rows, 60 steps 12.0 / 11.6 / 11.7 / 12.1; 718,146 rows, 30
+// steps 4.06 / 3.92 / 3.95 / 4.07; 2,587,018 rows, 60 steps 39.0 / 39.2 / 39.2 /
+// 39.6; 9,398,520 rows, 40 steps 71 each.
 int kept_columns(uint64_t n, bool cplx) {
   constexpr uint64_t kKeptPanelBytes = 48ull << 20;
   return static_cast<int>(std::min<uint64_t>(kKeptPanelBytes / (n * (cplx ? 16 : 8)), 1u << 20));
@@ -1313,11 +1317,6 @@ void* BlockOps::workspace(int slot, size_t bytes) {
     b.allocate(bytes);
   }
   return b.get();
-}
-
-void BlockOps::release_workspace() {
-  QMBED_CUDA(cudaStreamSynchronize(stream_));
-  workspace_.clear();
 }
 
 void BlockOps::ensure_partials(size_t doubles) {

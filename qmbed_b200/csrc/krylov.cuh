@@ -14,11 +14,11 @@ namespace qmbed {
 
 using C64 = std::complex<double>;
 
-// row_ptr = exclusive scan of per-row counts (u32 when the total fits).
 // False when QMBED_DENSE=scalar selects the CUDA-core kernels for the dense
 // contractions (block Gram, Ritz combinations) instead of the FP64 tensor cores.
 bool dense_on_tensor_cores();
 
+// row_ptr = exclusive scan of per-row counts (u32 when the total fits).
 uint64_t exclusive_scan_counts(const uint32_t* counts, uint64_t n, DeviceBuffer& row_ptr, bool* is64);
 C64 device_sum_complex(const double* interleaved, uint64_t n);
 double device_max_shifted_column(const double* diag, const double* offsum, uint64_t n, C64 shift);
@@ -86,7 +86,6 @@ class BlockOps {
   // Reference LCG start vector (deterministic_start, src/solve/mod.rs:729-742),
   // unnormalised, real part only; imaginary parts zero for complex vectors.
   void lcg_start(void* out, uint64_t n, uint64_t seed, int precision, bool cplx);
-  // r = y - lambda x; returns ||r||  (FP64 accumulation).
   // Normalises `count` Ritz candidates (columns of C, FP64) and their actions
   // (CA) in one launch and reads their norms before, Ritz values, residual
   // norms and norms after. False, with nothing done, for columns too long for
@@ -95,14 +94,15 @@ class BlockOps {
     double norm, value, residual, norm_after;
   };
   bool ritz_candidates(double* C, double* CA, uint64_t n, int count, bool cplx, std::vector<RitzCandidate>& out);
+  // r = y - lambda x; returns ||r||  (FP64 accumulation).
   double residual_norm(const void* y, const void* x, double lambda, uint64_t n, int precision, bool cplx);
   void sync();
 
   // Device buffer `slot` of at least `bytes`, kept for later calls on this
   // handle (grown, never shrunk) so that repeated solves reuse their blocks,
-  // like the reference EigshWorkspace (src/solve/mod.rs:477-526).
+  // like the reference EigshWorkspace (src/solve/mod.rs:477-526). Slots: 0-9
+  // the filtered solver, 10 projected eigenproblems.
   void* workspace(int slot, size_t bytes);
-  void release_workspace();
 
  private:
   // One queued step, its record on the device. The fused kernel makes the second

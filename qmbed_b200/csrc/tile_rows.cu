@@ -43,7 +43,7 @@ struct RowPair {  // diagonal products of two sites
 struct FillArgs {
   SectorParams p;
   uint64_t mask, dim;
-  int direct, colex;
+  int direct;
   const uint64_t* states;
   const uint16_t* orbits;
   const uint64_t* binom;
@@ -743,7 +743,6 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
   a.mask = low_mask<uint64_t>(p.sites);
   a.dim = n;
   a.direct = basis.direct() ? 1 : 0;
-  a.colex = basis.colex() ? 1 : 0;
   a.states = static_cast<const uint64_t*>(basis.states());
   a.orbits = basis.orbits();
   a.binom = basis.binomials();
@@ -834,6 +833,7 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
     if (distinct > kMaxStoredValues || static_cast<uint64_t>(distinct) > (1ull << (32 - col_bits))) return false;
   }
   out.n = n;
+  out.sms = sms;
   out.complex_values = cplx;
   out.col_bits = col_bits;
   out.codes = static_cast<int>(codes);
@@ -844,11 +844,11 @@ bool assemble_tile_rows(const SpinBasis& basis, const FlipProgram& prog, bool re
 
 namespace {
 
-// Sectors below this many tiles take four warps per tile: with one warp each,
+// Sectors of up to this many tiles per SM take four warps per tile: with one warp each,
 // fewer than eight warps would sit on an SM and a row's gathers run in series
 // (complex rows of 22 sites, 1003 tiles: 6.8 against 8.4 us a call; at 1776
 // tiles, 24 sites, 7.2 against 6.8).
-constexpr uint64_t kSplitTiles = 148 * 8;
+constexpr uint64_t kSplitTilesPerSm = 8;
 // Real FP64 rows keep eight gathers in flight per lane from here on: at 28
 // sites (718,146 rows) four take 20.8 us and eight 21.8, at 30 (2,587,018) 75.0
 // and 70.3, at 31 131.5 and 119.2. In FP32 and with complex vectors four are
@@ -870,7 +870,7 @@ void launch_spmv(const TileRows& rows, const SpinBasis& basis, const double* sqr
   constexpr int kWarps = kSpmvThreads / 32;
   const uint64_t blocks = (tiles + kWarps - 1) / kWarps;
   constexpr int kDeep = !VC && sizeof(T) == 8 ? 8 : 4;
-  if (tiles <= kSplitTiles) launch(tile_spmv_kernel<T, VC, VALC, VEC2, kWarps, 4>, tiles);
+  if (tiles <= kSplitTilesPerSm * rows.sms) launch(tile_spmv_kernel<T, VC, VALC, VEC2, kWarps, 4>, tiles);
   else if (rows.n >= kDeepRows) launch(tile_spmv_kernel<T, VC, VALC, VEC2, 1, kDeep>, blocks);
   else launch(tile_spmv_kernel<T, VC, VALC, VEC2, 1, 4>, blocks);
   QMBED_LAUNCH_CHECK();

@@ -12,7 +12,8 @@
 // with 0xffffffff in unused slots. The code tables hold the entry's value
 // without the orbit factor (block action, coordinates x / sqrt(R)) and divided
 // by sqrt(R_column) (y = H x), so neither action needs a scaled copy of x.
-// Transitions of a row that meet in one column stay separate entries.
+// Transitions of a row that meet in one column stay separate entries, or none
+// when they cancel.
 #pragma once
 
 #include <cstdint>
@@ -24,6 +25,7 @@ namespace qmbed {
 
 struct TileRows {
   uint64_t n = 0;
+  int sms = 0;              // of the device
   bool complex_values = false;
   int col_bits = 0, codes = 0;
   uint64_t nnz = 0;         // off-diagonal nonzeros after coalescing
