@@ -29,7 +29,7 @@ def test_exports_leave_nothing():
 @pytest.mark.parametrize("sector,cplx", [((14, 7, 3, None), True), ((14, 7, 0, 1), False), ((13, 6, None, -1), False)])
 @pytest.mark.parametrize("storage", ["packed", "explicit"])
 def test_the_count_before_an_export(sector, cplx, storage):
-    """The sizes of the arrays come from the tiles' own count: entries and nonzero diagonal values."""
+    """The sizes of the arrays: entries and nonzero diagonal values."""
     from qmbed_b200 import GpuBasis, GpuOperator, heisenberg_terms
     sites, up, momentum, parity = sector
     op = GpuOperator(GpuBasis(sites, up=up, momentum=momentum, parity=parity), heisenberg_terms(sites, j2=0.5, delta=0.7),
