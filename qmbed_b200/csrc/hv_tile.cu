@@ -1691,6 +1691,10 @@ const ImageTable* SpinBasis::build_image_table(bool required) const {
   QMBED_CUDA(cudaSetDevice(device_));
   size_t free_bytes = 0, total_bytes = 0;
   QMBED_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (bytes > free_bytes / 10 * 6) {  // idle blocks of earlier calls count as free
+    BlockPool::trim(device_);
+    QMBED_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  }
   if (bytes > free_bytes / 10 * 6) {
     if (required)
       raise(QMBED_UNSUPPORTED_BACKEND, "no image table for this sector: " + std::to_string(bytes) +
