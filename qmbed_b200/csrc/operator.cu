@@ -1355,7 +1355,13 @@ void SpinOperator::apply(int precision, bool complex_vectors, const void* x, voi
     const size_t bytes = vector_bytes(precision, cplx);
     if (basis_->symmetric() && overlap(x, y, bytes)) {
       void* copy = nullptr;
-      QMBED_CUDA(cudaMallocAsync(&copy, bytes, stream));
+      cudaError_t status = cudaMallocAsync(&copy, bytes, stream);
+      if (status == cudaErrorMemoryAllocation) {  // as DeviceBuffer::allocate
+        (void)cudaGetLastError();
+        BlockPool::trim(basis_->device());
+        status = cudaMallocAsync(&copy, bytes, stream);
+      }
+      QMBED_CUDA(status);
       QMBED_CUDA(cudaMemcpyAsync(copy, x, bytes, cudaMemcpyDeviceToDevice, stream));
       tile_spmv(*tile_, *basis_, inv_sqrt_.as<double>(), precision, cplx, copy, y, stream);
       QMBED_CUDA(cudaFreeAsync(copy, stream));
