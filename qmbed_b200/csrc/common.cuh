@@ -106,8 +106,8 @@ class DeviceBuffer {
 // Device blocks that finished calls leave for the next ones of the process (the
 // driver takes 0.1 to 5 ms per allocation and free): at most kLimit bytes per
 // device, the oldest freed first. They are given back before an allocation of
-// the library fails, and when the device's last handle with solver buffers is
-// gone. A block in here is idle: give() is called after the work on it has
+// the library fails or an image table is refused for lack of free memory, and
+// when the device's last handle with solver buffers is gone. A block in here is idle: give() is called after the work on it has
 // completed. Safe to use from several threads.
 class BlockPool {
  public:
